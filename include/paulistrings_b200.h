@@ -6,8 +6,9 @@
  * bytes per term) plus a coefficient column (float64 or float32), kept sorted by
  * key with unique keys.  All entry points take plain pointers and sizes; no
  * torch or CUDA types cross the boundary.  Every call returns a ps_status; on
- * any error the store keeps the last completed layer and ps_last_error()
- * describes the failure.  One handle per host thread; each handle issues its
+ * any error the store keeps the last completed layer (ps_propagate may take
+ * several layers of a small sum in one launch: they complete or fail together)
+ * and ps_last_error() describes the failure.  One handle per host thread; each handle issues its
  * work on its own CUDA stream.
  *
  * Reference interfaces replaced (paths inside lkdvos/paulistrings-rs):

@@ -16,6 +16,7 @@
 #include "ps_device.cuh"
 #include "ps_kernels.h"
 #include "ps_scorer.h"
+#include "ps_run.h"
 #include "ps_store.h"
 
 using namespace psb;
@@ -130,6 +131,11 @@ struct ps_sum {
     bool def_classified = false;
     bool def_flags = false;
     ps_layer_stats* def_stats = nullptr;
+    // A run of layers of a small sum in one launch (ps_run.cu): its program and noise tables, its
+    // control words, per-layer counts and block summaries, and their pinned host copies.
+    Buf run_prog, run_state, run_sums;
+    unsigned char* hrun = nullptr;        // pinned, hrun_cap bytes
+    size_t hrun_cap = 0;
     Buf noise_drops;                      // folded noise: own rows first dropped after channel j
     unsigned long long* hnoise = nullptr; // pinned, kMaxNoise + 1 words
     KeepProg clean_keep{};
@@ -909,6 +915,17 @@ uint64_t inherit_interval(const ps_policy* p, const ps_sum* s) {
     return p->passes[0].samples;
 }
 
+// A single-qubit key-preserving channel whose factors can be folded into the next layer: it
+// leaves the identity alone and shrinks no coefficient's magnitude by less than nothing
+// (|factor| <= 1), so the keep program passes after it only if it passed before it.
+bool foldable_noise(const ps_table& t, int nq) {
+    if (t.mode != PS_TABLE_LOCAL || t.k != 1 || t.num_entries != 1 || t.entries[0].local_delta != 0) return false;
+    if (t.qubits[0] >= (uint32_t)nq || t.entries[0].amplitude[0] != 1.0) return false;
+    for (int s = 1; s < 4; ++s)
+        if (!(std::fabs(t.entries[0].amplitude[s]) <= 1.0)) return false;
+    return true;
+}
+
 // ---------------------------------------------------------------------------
 // per-width / per-dtype operations
 // ---------------------------------------------------------------------------
@@ -1351,6 +1368,256 @@ struct Engine {
         cudaError_t e = spin_sync(s->stream);
         if (e != cudaSuccess) return cuda_fail(s, e, "apply: counts");
         return finish_deferred(s, s->hcount[22]);
+    }
+
+    // A run of layers on a small sum in one launch (ps_run.cu), from layer li of ps_propagate's
+    // tables.  *consumed: the channels it covered (0: none; the caller takes the next one layer by
+    // layer).  The run takes rotation-shaped and key-preserving tables with at most kRunLevels
+    // partner bits, any keep program and at most one plain TopN pass; layers the light-cone skip
+    // passes over and folded noise are resolved here as the per-layer path resolves them.  It is not used while per-kernel profiling or a
+    // failure injection is on (both act on the per-layer kernels).
+    static ps_status run_layers(ps_sum* s, const std::vector<ps_table>& tables, uint64_t li, const ps_policy* policy,
+                                uint64_t* terms_after, ps_run_stats* rs, uint64_t* consumed) {
+        *consumed = 0;
+        if (s->prof.events || s->fault_oom_after >= 0 || s->fault_stall || s->fault_flag) return PS_OK;
+        if (s->slotted || s->deferred || s->n == 0) return PS_OK;
+        const uint64_t n0 = s->n;
+        // The bound on the sum: the blocks must hold it with its partners, which can be as many; above
+        // half of what they hold the first layer could already end the run (f64, one word: 425,000
+        // of 845,000 rows).  Below it the run wins at every size measured (ps_run.cu).
+        uint64_t topn = 0;
+        if (policy && policy->num_passes > 0) {
+            const ps_pass& p = policy->passes[0];
+            if (policy->num_passes != 1 || p.kind != PS_PASS_TOPN || p.n == 0 || n0 > p.n) return PS_OK;
+            topn = p.n;
+        }
+        if (n0 > (uint64_t)kRunMaxBlocks * 65536 / 2) return PS_OK;
+        const uint32_t rcap = RunOps<W, T>::rows_per_block();
+        const int blocks = std::min(s->sms, kRunMaxBlocks);
+        const uint64_t room = (uint64_t)rcap * blocks;
+        if (n0 > room / 2) return PS_OK;
+        KeepProg keep;
+        std::string why;
+        ps_status ps = lower_keep(policy, keep, why);
+        if (ps != PS_OK) return set_err(s, ps, why);
+
+        // the program: one entry per launch layer or skipped channel
+        struct Entry {
+            uint64_t channels;  // channels it covers (folded noise first)
+            int32_t prog;       // place in the program, -1: skipped
+            bool partners;
+            uint64_t lsup[W];
+        };
+        std::vector<Entry> entries;
+        std::vector<RunLayer<W, T>> prog;
+        std::vector<T> noise_f;
+        std::vector<uint16_t> noise_q;
+        uint64_t sup[W];
+        for (int w = 0; w < W; ++w) sup[w] = s->support[w];
+        bool clean = s->support_known && s->keep_clean && std::memcmp(&keep, &s->clean_keep, sizeof keep) == 0;
+        const uint64_t end = std::min<uint64_t>(tables.size(), li + kRunMaxLayers);
+        uint64_t grow = n0;  // bound on the rows of the run
+        for (uint64_t c = li; c < end;) {
+            uint64_t fj = c;
+            while (fj < end && fj - c < (uint64_t)kMaxNoise && foldable_noise(tables[fj], s->nq)) ++fj;
+            Entry en{};
+            RotLayer<W> R;
+            bool general = false;
+            uint64_t at = c;
+            if (fj > c && fj < end) {  // folded into the rotation that follows, if one with partners does
+                if (to_rot_layer<W, T>(tables[fj], R, *s->levels, why, &general) == PS_OK && !general && R.partners &&
+                    s->levels->n <= kRunLevels)
+                    at = fj;
+            }
+            if (at == c) {
+                general = false;
+                if (to_rot_layer<W, T>(tables[c], R, *s->levels, why, &general) != PS_OK || general) break;
+                if (R.partners && s->levels->n > kRunLevels) break;
+                // noise cut off from its rotation by the end of the run is left to the next one
+                if (fj > c && fj == end && end < tables.size()) break;
+            }
+            table_support<W>(tables[at], en.lsup);
+            en.channels = at - c + 1;
+            en.partners = R.partners != 0;
+            en.prog = -1;
+            const bool identity0 = R.wide || ((T)R.a1[0] == T(0) && (T)R.a0[0] == T(1));
+            bool skip = at == c && identity0 && clean;
+            for (int w = 0; w < W; ++w) skip = skip && !(en.lsup[w] & sup[w]);
+            if (!skip) {
+                RunLayer<W, T> P;
+                std::memset(&P, 0, sizeof P);
+                for (int w = 0; w < W; ++w) {
+                    P.gx[w] = R.gx[w];
+                    P.gz[w] = R.gz[w];
+                }
+                for (int q = 0; q < 16; ++q) {
+                    P.a0[q] = std::is_same<T, double>::value ? (T)R.a0[q] : (T)R.a0f[q];
+                    P.a1[q] = std::is_same<T, double>::value ? (T)R.a1[q] : (T)R.a1f[q];
+                }
+                P.cos64 = R.cos64;
+                P.sin64 = R.sin64;
+                P.cos32 = R.cos32;
+                P.sin32 = R.sin32;
+                P.wide = R.wide;
+                P.partners = R.partners;
+                for (int q = 0; q < 2; ++q) {
+                    P.qw[q] = R.qw[q];
+                    P.qb[q] = R.qb[q];
+                }
+                P.pattern_mask = R.pattern_mask;
+                if (R.partners) {
+                    P.nlev = s->levels->n;
+                    for (int q = 0; q < s->levels->n; ++q) P.rank[q] = s->levels->rank[q];
+                }
+                P.noise_first = (int32_t)noise_q.size();
+                P.noise_n = (int32_t)(at - c);
+                for (uint64_t q = c; q < at; ++q) {
+                    noise_q.push_back((uint16_t)tables[q].qubits[0]);
+                    for (int z = 0; z < 4; ++z) noise_f.push_back((T)tables[q].entries[0].amplitude[z]);
+                }
+                en.prog = (int32_t)prog.size();
+                prog.push_back(P);
+                if (R.partners) {
+                    grow = std::min<uint64_t>(2 * grow, room);
+                    for (int w = 0; w < W; ++w) sup[w] |= en.lsup[w];
+                }
+                clean = s->support_known;
+            }
+            entries.push_back(en);
+            c = at + 1;
+        }
+        if (prog.empty()) return PS_OK;
+        uint64_t wcap = grow;
+        if (topn) wcap = std::min<uint64_t>(wcap, std::max<uint64_t>(topn, n0));
+
+        // buffers
+        const int spare = 1 - s->cur;
+        const uint64_t pcap = wcap;
+        const size_t nl = prog.size(), nd = noise_q.size();
+        auto up16 = [](size_t b) { return (b + 15) / 16 * 16; };
+        const size_t prog_b = up16(nl * sizeof(RunLayer<W, T>)), nf_b = up16(nd * 4 * sizeof(T)), nq_b = up16(nd * 2);
+        const size_t stats_b = up16((2 * nl + nd) * sizeof(unsigned int));
+        cudaError_t e = reserve_store(s, spare, wcap);
+        if (e == cudaSuccess) e = ensure(s, s->pk, pcap * kKeyBytes);
+        if (e == cudaSuccess) e = ensure(s, s->pc, pcap * sizeof(T));
+        if (e == cudaSuccess) e = ensure(s, s->run_prog, prog_b + nf_b + nq_b);
+        if (e == cudaSuccess) e = ensure(s, s->run_state, sizeof(RunState) + stats_b);
+        if (e == cudaSuccess) e = ensure(s, s->run_sums, kRunMaxBlocks * sizeof(RunSummary<W>));
+        const size_t head_b = offsetof(RunState, ties);
+        const size_t need = prog_b + nf_b + nq_b + up16(head_b) + stats_b + 16;
+        if (e == cudaSuccess && s->hrun_cap < need) {
+            if (s->hrun) cudaFreeHost(s->hrun);
+            s->hrun = nullptr;
+            s->hrun_cap = 0;
+            e = cudaMallocHost(&s->hrun, need + need / 2);
+            if (e == cudaSuccess) s->hrun_cap = need + need / 2;
+        }
+        if (e != cudaSuccess) return cuda_fail(s, e, "run: allocation");
+        if (s->hist_ready) {
+            cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
+            s->hist_ready = false;
+        }
+        std::memcpy(s->hrun, prog.data(), nl * sizeof(RunLayer<W, T>));
+        if (nd) {
+            std::memcpy(s->hrun + prog_b, noise_f.data(), nd * 4 * sizeof(T));
+            std::memcpy(s->hrun + prog_b + nf_b, noise_q.data(), nd * 2);
+        }
+        unsigned char* dprog = static_cast<unsigned char*>(s->run_prog.p);
+        unsigned char* dstate = static_cast<unsigned char*>(s->run_state.p);
+        cudaMemcpyAsync(dprog, s->hrun, prog_b + nf_b + nq_b, cudaMemcpyHostToDevice, s->stream);
+        cudaMemsetAsync(dstate, 0, sizeof(RunState) + stats_b, s->stream);
+        RunArgs<W, T> a;
+        std::memset(&a, 0, sizeof a);
+        a.Sk = K(s, s->cur);
+        a.Sc = C(s, s->cur);
+        a.n = n0;
+        a.Wk = K(s, spare);
+        a.Wc = C(s, spare);
+        a.wcap = wcap;
+        a.Pk = (uint64_t*)s->pk.p;
+        a.Pc = (T*)s->pc.p;
+        a.pcap = pcap;
+        a.prog = reinterpret_cast<const RunLayer<W, T>*>(dprog);
+        a.nlayers = (uint32_t)nl;
+        a.noise_f = reinterpret_cast<const T*>(dprog + prog_b);
+        a.noise_q = reinterpret_cast<const uint16_t*>(dprog + prog_b + nf_b);
+        a.keep = keep;
+        a.topn = topn;
+        // the last boundary's window, in the run's finer bins around its middle
+        a.window = topn && s->topn_window && s->topn_base ? 1 : 0;
+        a.window_base = a.window ? s->topn_base + (1024ull << 48) - (1024ull << 44) : 0;
+        a.sums = (RunSummary<W>*)s->run_sums.p;
+        a.st = reinterpret_cast<RunState*>(dstate);
+        a.out_rows = reinterpret_cast<unsigned int*>(dstate + sizeof(RunState));
+        a.after_rows = a.out_rows + nl;
+        a.drops = a.after_rows + nl;
+        a.ctl = s->ctl;
+        a.rcap = rcap;
+        e = RunOps<W, T>::launch(a, blocks, s->stream, &s->prof);
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+            cudaGetLastError();
+            return PS_OK;  // nothing ran: layer by layer
+        }
+        unsigned char* hhead = s->hrun + prog_b + nf_b + nq_b;
+        unsigned char* hstats = hhead + up16(head_b);
+        unsigned int* herr = reinterpret_cast<unsigned int*>(hstats + stats_b);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hhead, dstate, head_b, cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(hstats, dstate + sizeof(RunState), stats_b, cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(herr, &s->ctl->err, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess) e = spin_sync(s->stream);
+        if (e != cudaSuccess) return cuda_fail(s, e, "run");
+        ps = flags_status(s, herr[0], herr[1], "run");
+        if (ps != PS_OK) return ps;  // the input store is as it was
+        RunState head;
+        std::memcpy(&head, hhead, head_b);
+        const unsigned int* out_rows = reinterpret_cast<const unsigned int*>(hstats);
+        const unsigned int* after_rows = out_rows + nl;
+        const unsigned int* drops = after_rows + nl;
+
+        // what the per-layer path books after each layer
+        uint64_t n = n0, ci = li;
+        for (const Entry& en : entries) {
+            if (en.prog >= 0 && (unsigned int)en.prog >= head.layers_done) break;
+            if (en.prog < 0) {
+                rs->total_terms_in += n;
+                rs->skipped_terms_in += n;
+                ++rs->layers_skipped;
+                ++s->layers_skipped;
+                if (terms_after) terms_after[ci] = n;
+            } else {
+                const RunLayer<W, T>& P = prog[en.prog];
+                rs->total_terms_in += n;
+                for (int q = 0; q < P.noise_n; ++q) {
+                    n -= drops[P.noise_first + q];
+                    if (terms_after) terms_after[ci + q] = n;
+                    rs->total_terms_in += n;
+                }
+                if (out_rows[en.prog] > rs->peak_terms) rs->peak_terms = out_rows[en.prog];
+                n = topn ? after_rows[en.prog] : out_rows[en.prog];
+                if (terms_after) terms_after[ci + en.channels - 1] = n;
+                layer_done(s, en.lsup, keep, en.partners);
+            }
+            if (en.prog < 0 && n > rs->peak_terms) rs->peak_terms = n;
+            ci += en.channels;
+            rs->layers += en.channels;
+        }
+        *consumed = ci - li;
+        if (s->scorer) s->scorer_remaining -= (double)*consumed;
+        s->pre_valid = false;
+        s->nflag_valid = false;
+        if (head.layers_done == 0) return PS_OK;
+        s->f_valid = false;
+        if (n != head.n) return set_err(s, PS_ERR_DEVICE, "run: the rows do not match their count");
+        if (head.window) {
+            const uint64_t half = 1024ull << 48;
+            s->topn_window = true;
+            s->topn_base = head.boundary > half ? head.boundary - half : 0;
+        }
+        s->cur = spare;
+        s->n = n;
+        return PS_OK;
     }
 
     // The sort path: branch records, LSD radix sort of (key, record index), run-summing dedup
@@ -1892,17 +2159,6 @@ ps_status dispatch(ps_sum* s, F&& f) {
     return set_err(s, PS_ERR_UNSUPPORTED, "widths above 4 words (256 qubits) are not built");
 }
 
-// A single-qubit key-preserving channel whose factors can be folded into the next layer: it
-// leaves the identity alone and shrinks no coefficient's magnitude by less than nothing
-// (|factor| <= 1), so the keep program passes after it only if it passed before it.
-bool foldable_noise(const ps_table& t, int nq) {
-    if (t.mode != PS_TABLE_LOCAL || t.k != 1 || t.num_entries != 1 || t.entries[0].local_delta != 0) return false;
-    if (t.qubits[0] >= (uint32_t)nq || t.entries[0].amplitude[0] != 1.0) return false;
-    for (int s = 1; s < 4; ++s)
-        if (!(std::fabs(t.entries[0].amplitude[s]) <= 1.0)) return false;
-    return true;
-}
-
 // Would every layer pass of the policy leave a sum of the handle's current size (or smaller)
 // unchanged?  Then folding noise layers skips only passes that would have done nothing.
 bool passes_idle(const ps_policy* p, const ps_sum* s) {
@@ -1996,8 +2252,9 @@ ps_status ps_destroy(ps_sum* s) {
     if (!s) return PS_OK;
     DeviceGuard g(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (Buf* b : {&s->fcol[0], &s->fcol[1], &s->pf})
+    for (Buf* b : {&s->fcol[0], &s->fcol[1], &s->pf, &s->run_prog, &s->run_state, &s->run_sums})
         release(*b);
+    if (s->hrun) cudaFreeHost(s->hrun);
     for (Buf* b : {&s->keys[0], &s->keys[1], &s->coef[0], &s->coef[1], &s->pk, &s->pc, &s->idx, &s->dv, &s->fv,
                    &s->slots, &s->status, &s->bounds, &s->hist, &s->cand, &s->partial, &s->dout, &s->sort_status,
                    &s->up_x, &s->up_z, &s->up_c, &s->up_k, &s->up_v0, &s->up_v1, &s->up_c0, &s->up_st, &s->sel,
@@ -2102,6 +2359,16 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
     for (int i = 0; i < K_NUM_KERNELS; ++i) launches0 += s->prof.launches[i];
     const uint64_t collapses0 = s->collapses;
     for (uint64_t li = 0; li < num_channels; ++li) {
+        uint64_t ran = 0;
+        ps = dispatch<Engine>(s, [&](auto op) { return decltype(op)::run_layers(s, tables, li, policy, terms_after, &rs, &ran); });
+        if (ps != PS_OK) {
+            s->err = "layers from " + std::to_string(li) + ": " + s->err;
+            break;
+        }
+        if (ran) {
+            li += ran - 1;
+            continue;
+        }
         ps_layer_stats ls;
         // A run of single-qubit noise channels folds into the rotation layer that follows it:
         // their factors are applied, in order and with the keep program after each, to every term
@@ -2210,7 +2477,7 @@ ps_status ps_read_profile(ps_sum* s, ps_kernel_profile* out, int32_t cap, int32_
                                                 "k_merge",        "k_topn_hist",  "k_topn_step",  "k_topn_compact",
                                                 "k_pack",         "k_sort_hist",  "k_sort_pass",  "k_dedup",
                                                 "k_unpack",       "k_expect",     "k_gen_count",  "k_gen_branch",
-                                                "k_score",        "k_score_train"};
+                                                "k_score",        "k_score_train", "k_layer_run"};
     DeviceGuard g(s->device);
     s->prof.resolve();
     *count = K_NUM_KERNELS;

@@ -157,6 +157,7 @@ enum KernelId : int {
     K_GEN_BRANCH,
     K_SCORE,
     K_SCORE_TRAIN,
+    K_LAYER_RUN,  // k_layer_run: a run of rotation layers in one launch
     K_NUM_KERNELS
 };
 

@@ -55,40 +55,6 @@ constexpr int kScanTile = kBlock * kScanItems;
 constexpr int kApplyThreads = 512;  // k_level_apply block: 8 partners per thread
 static_assert(kScanTile == (int)kScanTileRows, "scan tile");
 
-// Does term k emit a partner?
-template <int W, typename T>
-__device__ __forceinline__ bool emits_partner(const RotLayer<W>& L, const AmpTab<T>& A, const uint64_t* k) {
-    if (L.wide) return anticommutes<W>(k, L.gx, L.gz);
-    return A.a1[pattern_of<W>(L, k)] != T(0);
-}
-
-// Own-row coefficient after the layer.
-template <int W, typename T>
-__device__ __forceinline__ T own_coeff(const RotLayer<W>& L, const AmpTab<T>& A, const uint64_t* k, T c) {
-    if (L.wide) return anticommutes<W>(k, L.gx, L.gz) ? mul_rn(c, Amp<T>::cs(L)) : c;
-    return mul_rn(c, A.a0[pattern_of<W>(L, k)]);
-}
-
-// Partner coefficient (DeltaEntry::emit / PreparedRotation::emit_generator).
-template <int W, typename T>
-__device__ __forceinline__ T partner_coeff(const RotLayer<W>& L, const AmpTab<T>& A, const uint64_t* k, T c) {
-    if (L.wide) {
-        uint32_t total = (1u + product_phase<W>(k, L.gx, L.gz)) & 3u;
-        T m = (total & 2u) ? -c : c;  // real mul_phase, coefficient.rs:107-114
-        return mul_rn(m, Amp<T>::sn(L));
-    }
-    return mul_rn(c, A.a1[pattern_of<W>(L, k)]);
-}
-
-// The folded noise channels, staged in shared memory (their factors are indexed by each lane's
-// pattern).
-template <typename T>
-struct NoiseSmem {
-    T f[kMaxNoise][4];
-    uint16_t q[kMaxNoise];
-    int n;
-};
-
 // The kernels that fold no noise take an empty argument in its place.
 struct NoNoise {};
 template <bool NOISE>
@@ -119,37 +85,6 @@ struct NoiseShared<T, false> {
     __device__ NoiseSmem<T>* tab() { return nullptr; }
     __device__ unsigned int* drops() { return nullptr; }
 };
-
-template <typename T>
-__device__ __forceinline__ void stage_noise(const NoiseList& N, NoiseSmem<T>& S) {
-    for (int i = threadIdx.x; i < N.n * 4; i += blockDim.x) {
-        if constexpr (std::is_same<T, double>::value)
-            S.f[i >> 2][i & 3] = N.f[i >> 2][i & 3];
-        else
-            S.f[i >> 2][i & 3] = N.ff[i >> 2][i & 3];
-    }
-    for (int i = threadIdx.x; i < N.n; i += blockDim.x) S.q[i] = N.q[i];
-    if (threadIdx.x == 0) S.n = N.n;
-}
-
-// The folded channels applied to coefficient v of key k in order, as the separate layers would:
-// a channel multiplies by its factor for k's pattern on its qubit (the identity's factor is 1,
-// skipped), then the term must stay nonzero and pass the keep program.  Returns the index of the
-// channel after which the term is dropped, or S.n when it survives all of them.
-template <int W, typename T>
-__device__ __forceinline__ int noise_apply(const NoiseSmem<T>& S, const KeepProg& keep, const uint64_t* k, T& v) {
-    if (!(v != T(0) && keep_eval<W>(keep, k, to_f64(v)))) return 0;
-    for (int j = 0; j < S.n; ++j) {
-        const int q = S.q[j];
-        const uint32_t s = (uint32_t)((pick<W>(k, q >> 6) >> (q & 63)) & 1u) |
-                           (uint32_t)((pick<W>(k, W + (q >> 6)) >> (q & 63)) & 1u) << 1;
-        if (s) {
-            v = mul_rn(v, S.f[j][s]);
-            if (!(v != T(0) && keep_eval<W>(keep, k, to_f64(v)))) return j;
-        }
-    }
-    return S.n;
-}
 
 // ---------------------------------------------------------------------------
 // k_classify: warp-striped (lane l of warp w reads row base_w + 32 i + l, coalesced 16W-byte
@@ -635,32 +570,6 @@ struct MergeSmem {
     static constexpr int F_SLOTS = TILE + 4 + 16;
     static constexpr size_t f_bytes = ((size_t)F_SLOTS * sizeof(float) + 15) / 16 * 16;
 };
-
-template <int W>
-__device__ __forceinline__ void ld_row(const uint64_t* base, uint32_t r, uint64_t (&k)[2 * W]) {
-    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(base + (size_t)r * 2 * W);
-#pragma unroll
-    for (int q = 0; q < W; ++q) {
-        ulonglong2 v = p[q];
-        k[2 * q] = v.x;
-        k[2 * q + 1] = v.y;
-    }
-}
-
-template <int W>
-__device__ __forceinline__ bool le_regs(const uint64_t (&a)[2 * W], const uint64_t (&b)[2 * W]) {
-#pragma unroll
-    for (int i = 0; i < 2 * W; ++i)
-        if (a[i] != b[i]) return a[i] < b[i];
-    return true;
-}
-template <int W>
-__device__ __forceinline__ bool eq_regs(const uint64_t (&a)[2 * W], const uint64_t (&b)[2 * W]) {
-    uint64_t d = 0;
-#pragma unroll
-    for (int i = 0; i < 2 * W; ++i) d |= a[i] ^ b[i];
-    return d == 0;
-}
 
 // Walk one thread's merge-path range once, with the two run heads held in registers (one
 // shared load per consumed item).  Own row first, partner second when their keys are equal, as

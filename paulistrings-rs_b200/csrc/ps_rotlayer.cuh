@@ -1,7 +1,11 @@
-// ps_rotlayer.cuh -- device helpers of a rotation layer's table shared by the layer kernels
-// and the TopN compaction that classifies its output rows for the next layer: support pattern
-// of a key, per-pattern amplitudes staged in shared memory, the partner test, divergence rank.
+// ps_rotlayer.cuh -- device helpers of a rotation layer's table shared by the layer kernels,
+// the kernel that runs many layers in one launch and the TopN compaction that classifies its
+// output rows for the next layer: support pattern of a key, per-pattern amplitudes staged in
+// shared memory, the partner test, own and partner coefficients, folded noise, divergence rank,
+// merge comparisons.  LT: RotLayer<W>, or a type with its fields.
 #pragma once
+
+#include <type_traits>
 
 #include "ps_device.cuh"
 #include "ps_kernels.h"
@@ -19,8 +23,8 @@ __device__ __forceinline__ uint64_t pick(const uint64_t* k, int wi) {
 }
 
 // support pattern of key k (LocalPtm::support_bits, channel/prepared.rs:141-151)
-template <int W>
-__device__ __forceinline__ uint32_t pattern_of(const RotLayer<W>& L, const uint64_t* k) {
+template <int W, typename LT>
+__device__ __forceinline__ uint32_t pattern_of(const LT& L, const uint64_t* k) {
     uint32_t s = (uint32_t)((pick<W>(k, L.qw[0]) >> L.qb[0]) & 1u) |
                  (uint32_t)((pick<W>(k, W + L.qw[0]) >> L.qb[0]) & 1u) << 1 |
                  (uint32_t)((pick<W>(k, L.qw[1]) >> L.qb[1]) & 1u) << 2 |
@@ -36,10 +40,10 @@ struct Amp<double> {
     __device__ static double a0(const RotLayer<W>& L, uint32_t s) { return L.a0[s]; }
     template <int W>
     __device__ static double a1(const RotLayer<W>& L, uint32_t s) { return L.a1[s]; }
-    template <int W>
-    __device__ static double cs(const RotLayer<W>& L) { return L.cos64; }
-    template <int W>
-    __device__ static double sn(const RotLayer<W>& L) { return L.sin64; }
+    template <typename LT>
+    __device__ static double cs(const LT& L) { return L.cos64; }
+    template <typename LT>
+    __device__ static double sn(const LT& L) { return L.sin64; }
 };
 template <>
 struct Amp<float> {
@@ -47,10 +51,10 @@ struct Amp<float> {
     __device__ static float a0(const RotLayer<W>& L, uint32_t s) { return L.a0f[s]; }
     template <int W>
     __device__ static float a1(const RotLayer<W>& L, uint32_t s) { return L.a1f[s]; }
-    template <int W>
-    __device__ static float cs(const RotLayer<W>& L) { return L.cos32; }
-    template <int W>
-    __device__ static float sn(const RotLayer<W>& L) { return L.sin32; }
+    template <typename LT>
+    __device__ static float cs(const LT& L) { return L.cos32; }
+    template <typename LT>
+    __device__ static float sn(const LT& L) { return L.sin32; }
 };
 
 // The layer's per-pattern amplitudes staged in shared memory: indexing the kernel-parameter
@@ -69,8 +73,8 @@ __device__ __forceinline__ void stage_amps(const RotLayer<W>& L, AmpTab<T>& t) {
     }
 }
 
-template <int W, typename T>
-__device__ __forceinline__ bool emits_partner_regs(const RotLayer<W>& L, const AmpTab<T>& A,
+template <int W, typename T, typename LT>
+__device__ __forceinline__ bool emits_partner_regs(const LT& L, const AmpTab<T>& A,
                                                    const uint64_t (&k)[2 * W]) {
     if (L.wide) {
         uint64_t f = 0;
@@ -90,6 +94,91 @@ __device__ __forceinline__ uint32_t div_regs(const uint64_t (&a)[2 * W], const u
         if (d) r = 64u * i + (uint32_t)__clzll((long long)d);
     }
     return r;
+}
+
+// Own-row coefficient after the layer.
+template <int W, typename T, typename LT>
+__device__ __forceinline__ T own_coeff(const LT& L, const AmpTab<T>& A, const uint64_t* k, T c) {
+    if (L.wide) return anticommutes<W>(k, L.gx, L.gz) ? mul_rn(c, Amp<T>::cs(L)) : c;
+    return mul_rn(c, A.a0[pattern_of<W>(L, k)]);
+}
+
+// Partner coefficient (DeltaEntry::emit / PreparedRotation::emit_generator).
+template <int W, typename T, typename LT>
+__device__ __forceinline__ T partner_coeff(const LT& L, const AmpTab<T>& A, const uint64_t* k, T c) {
+    if (L.wide) {
+        uint32_t total = (1u + product_phase<W>(k, L.gx, L.gz)) & 3u;
+        T m = (total & 2u) ? -c : c;  // real mul_phase, coefficient.rs:107-114
+        return mul_rn(m, Amp<T>::sn(L));
+    }
+    return mul_rn(c, A.a1[pattern_of<W>(L, k)]);
+}
+
+// The folded noise channels, staged in shared memory (their factors are indexed by each lane's
+// pattern).
+template <typename T>
+struct NoiseSmem {
+    T f[kMaxNoise][4];
+    uint16_t q[kMaxNoise];
+    int n;
+};
+
+template <typename T>
+__device__ __forceinline__ void stage_noise(const NoiseList& N, NoiseSmem<T>& S) {
+    for (int i = threadIdx.x; i < N.n * 4; i += blockDim.x) {
+        if constexpr (std::is_same<T, double>::value)
+            S.f[i >> 2][i & 3] = N.f[i >> 2][i & 3];
+        else
+            S.f[i >> 2][i & 3] = N.ff[i >> 2][i & 3];
+    }
+    for (int i = threadIdx.x; i < N.n; i += blockDim.x) S.q[i] = N.q[i];
+    if (threadIdx.x == 0) S.n = N.n;
+}
+
+// The folded channels applied to coefficient v of key k in order, as the separate layers would:
+// a channel multiplies by its factor for k's pattern on its qubit (the identity's factor is 1,
+// skipped), then the term must stay nonzero and pass the keep program.  Returns the index of the
+// channel after which the term is dropped, or S.n when it survives all of them.
+template <int W, typename T>
+__device__ __forceinline__ int noise_apply(const NoiseSmem<T>& S, const KeepProg& keep, const uint64_t* k, T& v) {
+    if (!(v != T(0) && keep_eval<W>(keep, k, to_f64(v)))) return 0;
+    for (int j = 0; j < S.n; ++j) {
+        const int q = S.q[j];
+        const uint32_t s = (uint32_t)((pick<W>(k, q >> 6) >> (q & 63)) & 1u) |
+                           (uint32_t)((pick<W>(k, W + (q >> 6)) >> (q & 63)) & 1u) << 1;
+        if (s) {
+            v = mul_rn(v, S.f[j][s]);
+            if (!(v != T(0) && keep_eval<W>(keep, k, to_f64(v)))) return j;
+        }
+    }
+    return S.n;
+}
+
+// Rows of a staged run in shared memory and comparisons on keys held in registers.
+template <int W>
+__device__ __forceinline__ void ld_row(const uint64_t* base, uint32_t r, uint64_t (&k)[2 * W]) {
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(base + (size_t)r * 2 * W);
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        ulonglong2 v = p[q];
+        k[2 * q] = v.x;
+        k[2 * q + 1] = v.y;
+    }
+}
+
+template <int W>
+__device__ __forceinline__ bool le_regs(const uint64_t (&a)[2 * W], const uint64_t (&b)[2 * W]) {
+#pragma unroll
+    for (int i = 0; i < 2 * W; ++i)
+        if (a[i] != b[i]) return a[i] < b[i];
+    return true;
+}
+template <int W>
+__device__ __forceinline__ bool eq_regs(const uint64_t (&a)[2 * W], const uint64_t (&b)[2 * W]) {
+    uint64_t d = 0;
+#pragma unroll
+    for (int i = 0; i < 2 * W; ++i) d |= a[i] ^ b[i];
+    return d == 0;
 }
 
 }  // namespace psb
