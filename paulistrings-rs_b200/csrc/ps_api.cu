@@ -16,6 +16,7 @@
 #include "ps_device.cuh"
 #include "ps_kernels.h"
 #include "ps_scorer.h"
+#include "ps_cut.h"
 #include "ps_run.h"
 #include "ps_store.h"
 
@@ -114,7 +115,7 @@ struct ps_sum {
     bool pre_valid = false;
     const ps_table* pre_table = nullptr;
     uint64_t pre_n = 0;
-    // the merge before such a TopN pass: each output row's partner test under next_table
+    // the merge before such a TopN pass: each output row's partner test (a byte) under next_table
     Buf nflag;
     bool nflag_valid = false;
     const ps_table* nflag_table = nullptr;
@@ -126,7 +127,8 @@ struct ps_sum {
     bool in_propagate = false;
     bool deferred = false;
     int def_prev_cur = 0;
-    uint64_t def_n_in = 0;
+    uint64_t def_n_in = 0;     // the input's rows (its slots' span)
+    uint64_t def_rows_in = 0;  // rows read
     int def_nlv = 0;
     bool def_classified = false;
     bool def_flags = false;
@@ -148,7 +150,23 @@ struct ps_sum {
     bool slotted = false;
     uint64_t live_n = 0;
     uint32_t slot_rows = 0;
-    Buf slot_count;
+    Buf slot_count[2];  // per store buffer
+    // A TopN cut left the rows in their slots (ps_cut.h): a row is live iff its select key is above
+    // cut_boundary, or equal to it and not after row cut_last_tie, cut_rows rows in all, live_n of them live, and the partners of
+    // the table cut_table are listed (nullptr: the lists do not hold).  Only inside ps_propagate,
+    // between a layer and the next; any other reader compacts first (Engine::densify).
+    bool cut = false;
+    unsigned long long cut_boundary = 0, cut_above = 0;
+    uint32_t cut_last_tie = 0;
+    uint64_t cut_rows = 0, cut_m = 0;
+    const ps_table* cut_table = nullptr;
+    bool cut_hist = false;          // the merge's histogram is in the cut's window
+    uint64_t topn_last = 0;         // the last TopN boundary (full-range select key; 0: none)
+    uint64_t excess_out = 0, excess_cap = 0;  // rows before the last TopN pass, and its budget
+    Buf cut_tiles, cut_blocks, cut_plist, cut_D, cut_cand, cut_state, cut_pr, cut_bslot;
+    bool def_cut = false;           // the deferred layer read a cut store (restored if it fails)
+    uint64_t def_live_n = 0;
+    uint32_t def_slot_rows = 0;
     std::string err;
 };
 
@@ -907,6 +925,9 @@ void table_support(const ps_table& t, uint64_t (&out)[W]) {
         if (t.qubits[j] < 64u * W) out[t.qubits[j] / 64] |= 1ull << (t.qubits[j] % 64);
 }
 
+// Terms of the handle's sum.
+uint64_t terms_of(const ps_sum* s) { return s->slotted ? s->live_n : s->n; }
+
 // The rescore interval of an inherited scored pass (the policy's first and only pass is a
 // scored TopN whose `samples` field is above 1, with a residual scorer attached), else 0.
 uint64_t inherit_interval(const ps_policy* p, const ps_sum* s) {
@@ -1002,7 +1023,7 @@ struct Engine {
         const int spare = 1 - s->cur;
         if (n == 0) {
             s->n = 0;
-            s->slotted = false;
+            s->slotted = s->cut = false;
             for (int w = 0; w < W; ++w) s->support[w] = 0;
             s->support_known = true;
             s->keep_clean = false;
@@ -1064,7 +1085,7 @@ struct Engine {
         }
         s->cur = spare;
         s->n = out_n;
-        s->slotted = false;
+        s->slotted = s->cut = false;
         if (s->hist_ready) {
             cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
             s->hist_ready = false;
@@ -1084,7 +1105,8 @@ struct Engine {
         uint64_t out_n = 0;
         e = StoreOps<W, T>::densify(K(s, s->cur), C(s, s->cur), s->n, slot_map(s), K(s, spare), C(s, spare),
                                     (unsigned long long*)s->status.p, s->ctl, s->hcount, &out_n, s->stream, &s->prof,
-                                    s->f_valid ? F(s, s->cur) : nullptr, s->f_valid ? F(s, spare) : nullptr);
+                                    s->f_valid ? F(s, s->cur) : nullptr, s->f_valid ? F(s, spare) : nullptr,
+                                    s->cut ? s->cut_boundary : 0ull, s->cut_above, s->live_n);
         s->prof.resolve();
         if (e != cudaSuccess) return cuda_fail(s, e, what);
         unsigned int fl = 0, fi = 0;
@@ -1094,12 +1116,12 @@ struct Engine {
         if (out_n != s->live_n) return set_err(s, PS_ERR_DEVICE, std::string(what) + ": slotted store lost rows");
         s->cur = spare;
         s->n = out_n;
-        s->slotted = false;
+        s->slotted = s->cut = false;
         return PS_OK;
     }
 
     static SlotMap slot_map(const ps_sum* s) {
-        return s->slotted ? SlotMap{(const unsigned int*)s->slot_count.p, s->slot_rows} : SlotMap{nullptr, 0u};
+        return s->slotted ? SlotMap{(const unsigned int*)s->slot_count[s->cur].p, s->slot_rows} : SlotMap{nullptr, 0u};
     }
 
     static ps_status download(ps_sum* s, uint64_t* x, uint64_t* z, double* c, uint64_t cap, uint64_t* nout) {
@@ -1146,7 +1168,9 @@ struct Engine {
         s->pre_valid = false;
         ps_status ps = lower_keep(policy, keep, why);
         if (ps != PS_OK) return set_err(s, ps, why);
-        if ((ps = densify(s, "apply")) != PS_OK) return ps;
+        // a store that the last TopN pass cut in place for this layer is read where it is
+        const bool cut_in = s->cut && s->cut_table == &t && s->in_propagate && !noise;
+        if (!cut_in && (ps = densify(s, "apply")) != PS_OK) return ps;
         RotationArgs<W, T> a;
         std::memset(&a, 0, sizeof a);
         bool general = false;
@@ -1164,10 +1188,10 @@ struct Engine {
                 return PS_OK;
             }
         }
-        const uint64_t n = s->n;
+        const uint64_t n = cut_in ? s->cut_rows : s->n;
         if (n >= (1ull << 31) - 1) return set_err(s, PS_ERR_UNSUPPORTED, "apply: at most 2^31 - 2 terms");
         const int spare = 1 - s->cur;
-        const uint64_t out_rows = a.L.partners ? 2 * n : n;
+        const uint64_t out_rows = cut_in ? n + s->cut_m : a.L.partners ? 2 * n : n;
         // the first layer pass is TopN (or ApproxTopN) and could trigger: the merge builds its
         // first select digit (the octave histogram); before plain TopN the merge writes slots
         const int first_pass = policy && policy->num_passes > 0 ? policy->passes[0].kind : PS_PASS_NONE;
@@ -1185,7 +1209,7 @@ struct Engine {
         if (e == cudaSuccess && carry_f) e = reserve_f(s, spare);
         if (e == cudaSuccess && carry_f && a.L.partners) e = ensure(s, s->pf, n * sizeof(float));
         if (e == cudaSuccess && slotted)
-            e = ensure(s, s->slot_count, (span_rows / merge_slot_rows<W>() + 1) * sizeof(unsigned int));
+            e = ensure(s, s->slot_count[spare], (span_rows / merge_slot_rows<W>() + 1) * sizeof(unsigned int));
         if (e != cudaSuccess) return cuda_fail(s, e, "apply: output store");
         // a plain TopN pass alone follows and a rotation layer (with partners) comes next: the
         // merge also writes each output row's partner test under that layer, for the compaction
@@ -1196,17 +1220,50 @@ struct Engine {
             bool general_next = false;
             if (to_rot_layer<W, T>(*s->next_table, a.next_L, *s->levels_next, why_next, &general_next) == PS_OK &&
                 !general_next && a.next_L.partners) {
-                if ((e = ensure(s, s->nflag, span_rows)) != cudaSuccess) return cuda_fail(s, e, "apply: partner flags");
+                if ((e = ensure(s, s->nflag, span_rows / merge_slot_rows<W>() * flag_stride(merge_slot_rows<W>()))) !=
+                    cudaSuccess) return cuda_fail(s, e, "apply: partner flags");
                 a.next_flags = static_cast<uint8_t*>(s->nflag.p);
                 s->nflag_valid = true;
                 s->nflag_table = s->next_table;
             }
         }
+        // ... and when the store also shall stay in its slots after that pass, it bins the select's first
+        // digit in the cut's finer window
+        CutArgs<W, T> cin;
+        if (cut_in) {
+            std::memset(&cin, 0, sizeof cin);
+            cin.keys = K(s, s->cur);
+            cin.coef = C(s, s->cur);
+            cin.count = (const unsigned int*)s->slot_count[s->cur].p;
+            cin.slot_rows = s->slot_rows;
+            cin.tiles = (CutTile*)s->cut_tiles.p;
+            cin.blocks = (CutBlock*)s->cut_blocks.p;
+            cin.plist = (uint16_t*)s->cut_plist.p;
+            cin.D = (uint16_t*)s->cut_D.p;
+            cin.ctl = s->ctl;
+            cin.next.n = s->levels->n;
+            for (int q = 0; q < s->levels->n && q < kCutLevels; ++q) cin.next.rank[q] = s->levels->rank[q];
+            const uint64_t slots = s->n / s->slot_rows;
+            a.cut = &cin;
+            a.cut_tiles = (uint32_t)slots;
+            a.cut_m = s->cut_m;
+            a.cut_boundary = s->cut_boundary;
+            a.cut_last_tie = s->cut_last_tie;
+            if ((e = ensure(s, s->cut_pr, (slots + 1) * sizeof(uint32_t))) != cudaSuccess ||
+                (e = ensure(s, s->cut_bslot, (out_rows / kMinTileRows + 4) * sizeof(uint4))) != cudaSuccess)
+                return cuda_fail(s, e, "apply: scratch");
+            a.cut_pr = (uint32_t*)s->cut_pr.p;
+            a.cut_bslot = (uint4*)s->cut_bslot.p;
+        }
         const uint64_t tiles_hi = out_rows / kMinTileRows + 4;
         if ((e = ensure(s, s->status, tiles_hi * sizeof(unsigned long long))) != cudaSuccess ||
             (e = ensure(s, s->bounds, (tiles_hi + 2) * sizeof(ulonglong2))) != cudaSuccess)
             return cuda_fail(s, e, "apply: scratch");
-        if (a.L.partners) {
+        if (cut_in) {
+            if ((e = ensure(s, s->pk, s->cut_m * kKeyBytes)) != cudaSuccess ||
+                (e = ensure(s, s->pc, s->cut_m * sizeof(T))) != cudaSuccess)
+                return cuda_fail(s, e, "apply: partner scratch");
+        } else if (a.L.partners) {
             if ((e = ensure(s, s->pk, n * kKeyBytes)) != cudaSuccess || (e = ensure(s, s->pc, n * sizeof(T))) != cudaSuccess ||
                 (e = ensure(s, s->idx, n * 4)) != cudaSuccess || (e = ensure(s, s->dv, n * 2)) != cudaSuccess ||
                 (e = ensure(s, s->fv, n * 4)) != cudaSuccess ||
@@ -1216,7 +1273,7 @@ struct Engine {
         a.Sk = K(s, s->cur);
         a.Sc = C(s, s->cur);
         a.n = n;
-        a.preclassified = preclassified && a.L.partners && !noise ? 1 : 0;
+        a.preclassified = cut_in || (preclassified && a.L.partners && !noise) ? 1 : 0;
         a.levels = s->levels;
         a.keep = keep;
         a.idx = (uint32_t*)s->idx.p;
@@ -1227,7 +1284,7 @@ struct Engine {
         a.bounds = (ulonglong2*)s->bounds.p;
         a.Pk = (uint64_t*)s->pk.p;
         a.Pc = (T*)s->pc.p;
-        a.p_cap = a.L.partners ? n : 0;
+        a.p_cap = cut_in ? s->cut_m : a.L.partners ? n : 0;
         a.Ok = K(s, spare);
         a.Oc = C(s, spare);
         a.out_cap = s->cap[spare];
@@ -1257,7 +1314,7 @@ struct Engine {
         a.stall_limit = s->fault_stall ? s->stall_limit : 0;
         s->fault_stall = false;
         uint64_t span = 0;
-        a.slot_count = slotted ? (unsigned int*)s->slot_count.p : nullptr;
+        a.slot_count = slotted ? (unsigned int*)s->slot_count[spare].p : nullptr;
         a.sms = s->sms;
         a.span_out = &span;
         if (noise && noise->n > 0) {
@@ -1281,6 +1338,20 @@ struct Engine {
                            policy->passes[0].n > 0 && !a.noise && a.L.partners &&
                            StoreOps<W, T>::cooperative_select();
         if (defer) a.defer_counts = s->hcount + 32;
+        // Cut in place rather than compacted: the pass reads the merge's partner tests, its window is
+        // known, and the last pass of this budget dropped at most a quarter.  The line: at 2^25 terms the
+        // cut saves 374 of 747 us a layer, and the merge pays 160 for reading the slots with 6 % of their
+        // rows dead, about 5 of them for each percent; layers of random angles drop 5 % in the middle and
+        // 11 % in the ninth decile, and a quarter keeps well below the 45 % where the two would be even.
+        s->cut_hist = false;
+        if (defer && a.next_flags && (s->topn_last >> 32) > (uint64_t)kCutReach + kCutMid && s->levels_next->n <= kCutLevels &&
+            span_rows < (1ull << 31) && policy->passes[0].n < (1ull << 31) &&
+            s->excess_cap == policy->passes[0].n && s->excess_out <= s->excess_cap + s->excess_cap / 4 &&
+            !skips_next(s, lsup, keep, a.next_L)) {
+            s->cut_hist = true;
+            a.topn_hist_mode = 5;
+            a.topn_hist_base = cut_base(s->topn_last);
+        }
         a.inject_flag = s->fault_flag;
         s->fault_flag = 0;
         s->deferred = false;
@@ -1294,7 +1365,7 @@ struct Engine {
         }
         s->hist_ready = fuse_topn;
         s->hist_kind = first_pass;
-        s->hist_window = fuse_topn && window;
+        s->hist_window = fuse_topn && window && !s->cut_hist;
         s->hist_base = a.topn_hist_base;
         uint64_t n_rot = n;  // terms entering the rotation, after the folded noise
         if (a.noise) {
@@ -1314,7 +1385,11 @@ struct Engine {
             // counts, statistics and the error check come with the TopN pass's synchronization
             s->deferred = true;
             s->def_prev_cur = s->cur;
-            s->def_n_in = n;
+            s->def_cut = s->cut;
+            s->def_live_n = s->live_n;
+            s->def_slot_rows = s->slot_rows;
+            s->def_n_in = s->n;
+            s->def_rows_in = n;
             s->def_nlv = s->levels->n;
             s->def_classified = !a.preclassified;
             s->def_flags = a.next_flags != nullptr;
@@ -1323,6 +1398,7 @@ struct Engine {
         }
         s->cur = spare;
         s->n = slotted ? span : out_n;  // deferred: a bound on the span
+        s->cut = false;
         s->slotted = slotted;
         s->live_n = out_n;              // deferred: not known yet
         s->slot_rows = slotted ? merge_slot_rows<W>() : 0u;
@@ -1341,17 +1417,19 @@ struct Engine {
         if (f[0]) {
             s->cur = s->def_prev_cur;
             s->n = s->def_n_in;
-            s->slotted = false;
-            s->live_n = 0;
+            s->slotted = s->cut = s->def_cut;
+            s->live_n = s->def_live_n;
+            s->slot_rows = s->def_slot_rows;
+            s->cut_table = nullptr;
             cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);  // the pass left it
             s->hist_ready = false;
             return flags_status(s, f[0], f[1], "apply");
         }
         const uint64_t m = c[0], out = c[1];
-        book_rotation_bytes<W, T>(&s->prof, s->def_n_in, m, out, s->def_nlv, s->def_classified);
+        book_rotation_bytes<W, T>(&s->prof, s->def_rows_in, m, out, s->def_nlv, s->def_classified);
         if (s->def_flags) s->prof.add_bytes(K_MERGE, (double)out);  // the partner-test bytes
         if (s->def_stats) {
-            s->def_stats->terms_in = s->def_n_in;
+            s->def_stats->terms_in = s->def_cut ? s->def_live_n : s->def_n_in;
             s->def_stats->partners = m;
             s->def_stats->terms_out = out;
             s->def_stats->terms_after_passes = out;
@@ -1359,7 +1437,20 @@ struct Engine {
         }
         s->n = span;
         s->live_n = out;
+        s->excess_out = out;
         return PS_OK;
+    }
+
+    // Would the next layer be passed over by the light-cone skip, once this one has run?
+    static bool skips_next(const ps_sum* s, const uint64_t (&lsup)[W], const KeepProg& keep, const RotLayer<W>& next) {
+        const bool identity0 = next.wide || ((T)next.a1[0] == T(0) && (T)next.a0[0] == T(1));
+        if (!identity0 || !s->support_known) return false;
+        (void)keep;  // this layer runs with it
+        uint64_t nsup[W];
+        table_support<W>(*s->next_table, nsup);
+        for (int w = 0; w < W; ++w)
+            if (nsup[w] & (s->support[w] | lsup[w])) return false;
+        return true;
     }
 
     // A deferred layer whose pass cannot run on the device's counts: wait for them here.
@@ -1614,6 +1705,7 @@ struct Engine {
             const uint64_t half = 1024ull << 48;
             s->topn_window = true;
             s->topn_base = head.boundary > half ? head.boundary - half : 0;
+            s->topn_last = head.boundary;
         }
         s->cur = spare;
         s->n = n;
@@ -1744,10 +1836,21 @@ struct Engine {
                 cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
                 ready = false;
             }
-            const bool use_hist = ready && i == 0;
+            bool use_hist = ready && i == 0;
             // the layer before did not wait for its counts: the select decides on the device
             // whether the live rows fit (the layer keeps a pass of n > 0 only, with its histogram)
-            const bool dfr = s->deferred && i == 0 && use_hist;
+            bool dfr = s->deferred && i == 0 && use_hist;
+            s->excess_cap = p.n;
+            if (dfr && s->cut_hist) {
+                bool cut = false;
+                ps_status ps = cut_topn(s, p.n, &cut);
+                if (ps != PS_OK) return ps;
+                if (cut) continue;
+                // the boundary left the window or cuts its ties: select in full range and compact
+                dfr = false;
+                use_hist = false;
+            }
+            s->cut_hist = false;
             if (s->deferred && !dfr) {
                 ps_status ps = settle_deferred(s);
                 if (ps != PS_OK) return ps;
@@ -1761,7 +1864,7 @@ struct Engine {
             if (p.n == 0) {
                 if (use_hist) cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
                 s->n = 0;
-                s->slotted = false;
+                s->slotted = s->cut = false;
                 continue;
             }
             const int spare = 1 - s->cur;
@@ -1781,8 +1884,10 @@ struct Engine {
                 if (classify && e == cudaSuccess) e = ensure(s, s->dv, p.n * 2);
             }
             if (e != cudaSuccess) {
+                // the layer itself is done: its counts, if it did not wait for them
+                ps_status ps = dfr ? settle_deferred(s) : PS_OK;
                 if (use_hist) cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
-                return cuda_fail(s, e, "topn: scratch");
+                return ps != PS_OK ? ps : cuda_fail(s, e, "topn: scratch");
             }
             // the merge wrote the rows' partner tests under that layer
             const bool flags_ok = classify && i == 0 && s->slotted && s->nflag_valid && s->nflag_table == s->next_table;
@@ -1824,12 +1929,13 @@ struct Engine {
                     const uint64_t half = 1024ull << 48;
                     s->topn_window = boundary != 0;
                     s->topn_base = boundary > half ? boundary - half : 0;
+                    s->topn_last = boundary;
                     break;
                 }
             }
             s->cur = spare;
             s->n = out_n;
-            s->slotted = false;
+            s->slotted = s->cut = false;
             if (classify && !topn_unclassified(s->hcount)) {
                 s->pre_valid = true;
                 s->pre_table = s->next_table;
@@ -1837,6 +1943,91 @@ struct Engine {
             }
         }
         return result;
+    }
+
+    // The TopN pass of a deferred layer by a cut in place (ps_cut.h), with the layer's counts and error
+    // check.  *cut false: the cut could not serve the pass, whose store is the layer's slotted output
+    // with its counts known.
+    static ps_status cut_topn(ps_sum* s, uint64_t keep_n, bool* cut) {
+        *cut = false;
+        s->cut_hist = false;
+        const uint64_t bound = s->n;  // on the span
+        const uint32_t slots = (uint32_t)(bound / s->slot_rows) + 1;
+        const uint32_t G = (uint32_t)CutOps<W, T>::blocks(s->sms);
+        cudaError_t e = ensure(s, s->cut_tiles, (size_t)slots * sizeof(CutTile));
+        if (e == cudaSuccess) e = ensure(s, s->cut_blocks, G * sizeof(CutBlock));
+        if (e == cudaSuccess) e = ensure(s, s->cut_plist, bound * sizeof(uint16_t));
+        if (e == cudaSuccess) e = ensure(s, s->cut_D, bound * sizeof(uint16_t));
+        if (e == cudaSuccess) e = ensure(s, s->cut_cand, (size_t)kCutCand * (sizeof(uint64_t) + sizeof(uint32_t)));
+        if (e == cudaSuccess) e = ensure(s, s->cut_state, sizeof(CutState));
+        if (e != cudaSuccess) {
+            ps_status ps = settle_deferred(s);  // the layer itself is done
+            cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
+            return ps != PS_OK ? ps : cuda_fail(s, e, "topn: scratch");
+        }
+        CutArgs<W, T> c;
+        std::memset(&c, 0, sizeof c);
+        c.keys = K(s, s->cur);
+        c.coef = C(s, s->cur);
+        c.flags = static_cast<const uint8_t*>(s->nflag.p);
+        c.count = (const unsigned int*)s->slot_count[s->cur].p;
+        c.slot_rows = s->slot_rows;
+        RotLayer<W> next_L;
+        std::string why;
+        bool general = false;
+        ps_status ps = to_rot_layer<W, T>(*s->next_table, next_L, *s->levels_next, why, &general);
+        if (ps != PS_OK) return set_err(s, ps, why);  // (apply checked this table)
+        c.next.n = s->levels_next->n;
+        for (int q = 0; q < s->levels_next->n; ++q) c.next.rank[q] = s->levels_next->rank[q];
+        c.tiles = (CutTile*)s->cut_tiles.p;
+        c.blocks = (CutBlock*)s->cut_blocks.p;
+        c.plist = (uint16_t*)s->cut_plist.p;
+        c.D = (uint16_t*)s->cut_D.p;
+        c.hist = (unsigned int*)s->hist.p;
+        c.base = (uint32_t)s->hist_base;
+        c.keep_n = keep_n;
+        c.cand = (uint64_t*)s->cut_cand.p;
+        c.cand_row = reinterpret_cast<uint32_t*>(c.cand + kCutCand);
+        c.state = (CutState*)s->cut_state.p;
+        c.ctl = s->ctl;
+        cudaMemsetAsync(c.state, 0, sizeof(CutState), s->stream);
+        e = CutOps<W, T>::cut(c, s->sms, s->stream, &s->prof);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->hcount, &s->ctl->count[0], offsetof(Ctl, spin_limit), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->hcount + 22, &s->ctl->span, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->hcount + 24, c.state, sizeof(CutState), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess) e = spin_sync(s->stream);
+        s->prof.resolve();
+        if (e != cudaSuccess) return cuda_fail(s, e, "topn");
+        ps = finish_deferred(s, s->hcount[22]);
+        if (ps != PS_OK) return ps;
+        unsigned int fl = 0, fi = 0;
+        topn_flags(s->hcount, &fl, &fi);
+        ps = flags_status(s, fl, fi, "topn");
+        if (ps != PS_OK) {
+            cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
+            return ps;
+        }
+        CutState r;
+        std::memcpy(&r, s->hcount + 24, sizeof r);
+        s->prof.add_bytes(K_TOPN_HIST, (double)r.rows * (sizeof(T) + 1) + (double)r.partners * (16 * W + 4));
+        if (r.status != 0) return PS_OK;
+        s->cut = true;
+        s->cut_boundary = r.boundary;
+        s->cut_above = r.above;
+        s->cut_last_tie = r.last_tie;
+        s->cut_rows = r.rows;
+        s->cut_m = r.partners;
+        s->cut_table = s->next_table;
+        s->live_n = keep_n;
+        const uint64_t half = 1024ull << 48;
+        s->topn_last = r.boundary;
+        s->topn_window = true;
+        s->topn_base = r.boundary > half ? r.boundary - half : 0;
+        *cut = true;
+        return PS_OK;
     }
 
     // CollapseSample: above `cache` terms, a systematic resample of `samples` points.
@@ -1980,7 +2171,7 @@ struct Engine {
             drop_hist();
             if (keep_n == 0 && live > 0) {
                 s->n = 0;
-                s->slotted = false;
+                s->slotted = s->cut = false;
                 return PS_OK;
             }
             return densify(s, "scored TopN");
@@ -2048,7 +2239,7 @@ struct Engine {
         }
         s->cur = spare;
         s->n = out_n;
-        s->slotted = false;
+        s->slotted = s->cut = false;
         if (classify && !topn_unclassified(s->hcount)) {
             s->pre_valid = true;
             s->pre_table = s->next_table;
@@ -2162,7 +2353,7 @@ ps_status dispatch(ps_sum* s, F&& f) {
 // Would every layer pass of the policy leave a sum of the handle's current size (or smaller)
 // unchanged?  Then folding noise layers skips only passes that would have done nothing.
 bool passes_idle(const ps_policy* p, const ps_sum* s) {
-    const uint64_t n = s->slotted ? s->live_n : s->n;
+    const uint64_t n = terms_of(s);
     for (int i = 0; p && i < p->num_passes; ++i)
         if (p->passes[i].kind != PS_PASS_NONE && n > p->passes[i].n) return false;
     return true;
@@ -2258,7 +2449,9 @@ ps_status ps_destroy(ps_sum* s) {
     for (Buf* b : {&s->keys[0], &s->keys[1], &s->coef[0], &s->coef[1], &s->pk, &s->pc, &s->idx, &s->dv, &s->fv,
                    &s->slots, &s->status, &s->bounds, &s->hist, &s->cand, &s->partial, &s->dout, &s->sort_status,
                    &s->up_x, &s->up_z, &s->up_c, &s->up_k, &s->up_v0, &s->up_v1, &s->up_c0, &s->up_st, &s->sel,
-                   &s->cnorms, &s->cfirst, &s->slot_count, &s->noise_drops, &s->nflag})
+                   &s->cnorms, &s->cfirst, &s->slot_count[0], &s->slot_count[1], &s->noise_drops, &s->nflag,
+                   &s->cut_tiles, &s->cut_blocks, &s->cut_plist, &s->cut_D, &s->cut_cand, &s->cut_state, &s->cut_pr,
+                   &s->cut_bslot})
         release(*b);
     if (s->ctl) cudaFree(s->ctl);
     if (s->sort.hist) cudaFree(s->sort.hist);
@@ -2292,7 +2485,7 @@ ps_status ps_upload(ps_sum* s, const uint64_t* x, const uint64_t* z, const doubl
 
 ps_status ps_len(ps_sum* s, uint64_t* n) {
     if (!s || !n) return PS_ERR_INVALID;
-    *n = s->slotted ? s->live_n : s->n;
+    *n = terms_of(s);
     return PS_OK;
 }
 
@@ -2354,7 +2547,7 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
     s->in_propagate = true;
     ps_run_stats rs;
     std::memset(&rs, 0, sizeof rs);
-    rs.peak_terms = s->n;
+    rs.peak_terms = terms_of(s);
     unsigned long long launches0 = 0;
     for (int i = 0; i < K_NUM_KERNELS; ++i) launches0 += s->prof.launches[i];
     const uint64_t collapses0 = s->collapses;
@@ -2390,7 +2583,7 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
                 }
             }
             uint64_t after[kMaxNoise];
-            const uint64_t n0 = s->n;
+            const uint64_t n0 = terms_of(s);
             s->next_table = fj + 1 < num_channels ? &tables[fj + 1] : nullptr;
             ps = dispatch<Engine>(s, [&](auto op) { return decltype(op)::apply(s, tables[fj], policy, &ls, &N, after); });
             if (ps == PS_OK && s->scorer) s->scorer_remaining -= (double)(fj - li);  // the folded layers' count-downs
@@ -2410,13 +2603,13 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
             }
             rs.total_terms_in += after[fj - li - 1];
             if (ls.terms_out > rs.peak_terms) rs.peak_terms = ls.terms_out;
-            if (terms_after) terms_after[fj] = s->n;
+            if (terms_after) terms_after[fj] = terms_of(s);
             ++rs.layers;
             li = fj;
             continue;
         }
-        rs.total_terms_in += s->n;
-        const uint64_t skipped0 = s->layers_skipped, n_in = s->n;
+        rs.total_terms_in += terms_of(s);
+        const uint64_t skipped0 = s->layers_skipped, n_in = terms_of(s);
         s->next_table = li + 1 < num_channels ? &tables[li + 1] : nullptr;
         ps = ps_apply_layer(s, &tables[li], policy, &ls);
         if (s->layers_skipped != skipped0) {
@@ -2432,9 +2625,10 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
             break;
         }
         if (ls.terms_out > rs.peak_terms) rs.peak_terms = ls.terms_out;
-        if (terms_after) terms_after[li] = s->n;
+        if (terms_after) terms_after[li] = terms_of(s);
         ++rs.layers;
     }
+    s->cut_table = nullptr;
     s->pre_valid = false;
     s->nflag_valid = false;
     s->next_table = nullptr;
@@ -2446,7 +2640,7 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    rs.final_terms = s->n;
+    rs.final_terms = terms_of(s);
     rs.device_ms = ms;
     unsigned long long launches1 = 0;
     for (int i = 0; i < K_NUM_KERNELS; ++i) launches1 += s->prof.launches[i];

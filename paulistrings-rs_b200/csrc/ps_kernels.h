@@ -222,6 +222,9 @@ struct KernelProf {
     }
 };
 
+// Bytes of a tile's partner tests, one per row of its slot, read 16 at a time.
+__host__ __device__ inline uint32_t flag_stride(uint32_t slot_rows) { return (slot_rows + 15) / 16 * 16; }
+
 // A slotted store: row e is live when e % rows < count[e / rows] (tile e / rows of a slotted
 // merge wrote count[e / rows] rows at the start of its slot).  count == nullptr: every row
 // below n is live (a dense store).
@@ -229,6 +232,9 @@ struct SlotMap {
     const unsigned int* count;
     uint32_t rows;
 };
+
+template <int W, typename T>
+struct CutArgs;
 
 template <int W, typename T>
 struct RotationArgs {
@@ -259,12 +265,21 @@ struct RotationArgs {
     KernelProf* prof;
     unsigned int* topn_hist;  // when set, the merge histograms its outputs into 2048 bins:
     int topn_hist_mode;       // 0 select key >> 52, 1 octave of |c|^2 (ApproxTopN),
-    uint64_t topn_hist_base;  // 2 window_key(select key, topn_hist_base) >> 48
+    uint64_t topn_hist_base;  // 2 window_key(select key, topn_hist_base) >> 48, 5 cut_bin (ps_cut.h)
     int inject_stall;         // failure injection: the merge skips its first tile
     int preclassified;        // idx, D and count[0] already hold this layer's partner list (written
                               // by the TopN compaction before it): no classify pass
     RotLayer<W> next_L;       // with next_flags (slotted output only): the next rotation layer,
-    uint8_t* next_flags;      // and per output row whether it emits a partner under it
+    uint8_t* next_flags;      // and a byte per output row, whether it emits a partner under it
+    // An input that a TopN cut left in its slots (ps_cut.h): Sk / Sc are the slots, n their rows; the
+    // cut listed this layer's partners.  cut: the pass's arguments (nullptr: a dense input).
+    const CutArgs<W, T>* cut;
+    uint32_t cut_tiles;                // slots of the input
+    uint64_t cut_m;                    // partners listed
+    unsigned long long cut_boundary;
+    uint32_t cut_last_tie;             // CutState::last_tie
+    uint32_t* cut_pr;                  // cut_tiles + 1 words, filled here
+    uint4* cut_bslot;                  // merge tiles + 1
     unsigned int inject_flag;          // failure injection: error bits written after the kernels
     unsigned long long* defer_counts;  // pinned: when set, the counts and error words are copied here
                                        // and the launcher returns without waiting (slotted output: the

@@ -19,6 +19,8 @@
 //                backward min-scan (the lower half moves up by the upper half's
 //                size); the last batch writes each partner at its sorted slot;
 //   k_partition  merge-path split points (a warp per run of tiles, 32-way search);
+//   (after a TopN cut in place, ps_cut.h, k_cut_place and k_cut_partition take the place of the level
+//                scans and k_partition)
 //   k_merge      merge own rows and partners (TMA bulk copies into shared
 //                memory), sum equal keys, drop exact zeros and keep-program
 //                rejects, and write the tile at its look-back offset or, before
@@ -31,7 +33,9 @@
 #include <atomic>
 #include <type_traits>
 #include <cstddef>
+#include <cstring>
 
+#include "ps_cut.h"
 #include "ps_device.cuh"
 #include "ps_kernels.h"
 #include "ps_rotlayer.cuh"
@@ -60,9 +64,9 @@ struct NoNoise {};
 template <bool NOISE>
 using NoiseArg = typename std::conditional<NOISE, NoiseList, NoNoise>::type;
 
-// Before a TopN pass whose compaction lists the next rotation layer's partners: the merge
-// writes, per output row (slot layout), whether the row emits a partner under that layer, so the
-// compaction decides from one byte instead of reading the key twice.
+// Before a TopN pass that lists the next rotation layer's partners: the merge writes a byte per output
+// row (flag_stride a tile), whether the row emits a partner under that layer, so the pass finds them
+// without reading the keys.  (A bit per row by a ballot made the merge 8 % slower.)
 template <int W>
 struct NextFlagArg {
     RotLayer<W> L;
@@ -71,6 +75,17 @@ struct NextFlagArg {
 struct NoNextFlag {};
 template <int W, bool ON>
 using NextArg = typename std::conditional<ON, NextFlagArg<W>, NoNextFlag>::type;
+
+// An input whose rows a TopN cut left in their slots (ps_cut.h).
+struct CutIn {
+    const uint32_t* pr;     // rows before each slot
+    const uint4* bslot;     // per merge tile: the slot of its first row, the rows before it and to its end
+    uint32_t slot_rows;
+    CutLive live;           // (last_tie: a row in the slots)
+};
+struct NoCut {};
+template <bool ON>
+using CutArg = typename std::conditional<ON, CutIn, NoCut>::type;
 
 // Shared storage for the staged channels only in the kernels that fold noise.
 template <typename T, bool ON>
@@ -577,13 +592,14 @@ struct MergeSmem {
 // pair is consumed in one step, so STEPS = ITEMS + 1 unrolled steps cover it (the caller checks
 // that nothing is left).  Step s leaves its output in ok[s] / ov[s] and sets bit s of the
 // returned mask when the output is kept (nonzero and passing the keep program).
-template <int W, typename T, int STEPS, bool NOISE, bool HASF>
+template <int W, typename T, int STEPS, bool NOISE, bool HASF, bool CUT>
 __device__ __forceinline__ uint32_t merge_walk(const uint64_t* sSk, const T* sSc, const uint64_t* sPk, const T* sPc,
                                                uint32_t& i, uint32_t ie, uint32_t& j, uint32_t je,
                                                const RotLayer<W>& L, const AmpTab<T>& A, const KeepProg& keep,
                                                uint64_t (&ok)[STEPS][2 * W], T (&ov)[STEPS],
                                                const NoiseSmem<T>* NS, unsigned int* s_drop, const float* sSf,
-                                               const float* sPf, float (&of)[STEPS]) {
+                                               const float* sPf, float (&of)[STEPS],
+                                               const CutArg<CUT>& CI, const uint32_t& last_tie, uint32_t rank0) {
     uint32_t mask = 0;
     uint64_t a[2 * W], b[2 * W];
     if (i < ie) ld_row<W>(sSk, i, a);
@@ -606,6 +622,10 @@ __device__ __forceinline__ uint32_t merge_walk(const uint64_t* sSk, const T* sSc
                     } else {
                         v = own_coeff<W, T>(L, A, a, c);
                     }
+                } else if constexpr (CUT) {
+                    // a row below the last cut is no row: a zero, which its equal partner replaces
+                    const T c = sSc[i];
+                    v = CI.live.test(to_f64(c), rank0 + i, last_tie) ? own_coeff<W, T>(L, A, a, c) : T(0);
                 } else {
                     v = own_coeff<W, T>(L, A, a, sSc[i]);
                 }
@@ -628,7 +648,15 @@ __device__ __forceinline__ uint32_t merge_walk(const uint64_t* sSk, const T* sSc
     return mask;
 }
 
-template <int W, typename T, bool NOISE, bool HASF, bool NEXTF = false>
+// A merge tile: its split points and, on a cut store, the slot its rows start in and that slot's rows
+// (slot, first, end).
+struct MergeTile {
+    ulonglong2 b0, b1;
+    uint4 slot;
+    unsigned int tile;
+};
+
+template <int W, typename T, bool NOISE, bool HASF, bool NEXTF = false, bool CUT = false>
 __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t* __restrict__ Sk, const T* __restrict__ Sc,
                                                   uint64_t n, const uint64_t* __restrict__ Pk,
                                                   const T* __restrict__ Pc, const ulonglong2* __restrict__ bounds,
@@ -640,7 +668,8 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
                                                   long long stall_limit, const NoiseArg<NOISE> N,
                                                   unsigned long long* __restrict__ noise_drops,
                                                   const float* __restrict__ Sf, const float* __restrict__ Pf,
-                                                  float* __restrict__ Of, const NextArg<W, NEXTF> NX = {}) {
+                                                  float* __restrict__ Of, const NextArg<W, NEXTF> NX = {},
+                                                  const CutArg<CUT> CI = {}) {
     using SM = MergeSmem<W, T>;
     constexpr int ITEMS = RotTile<W>::kMergeItems;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -648,7 +677,11 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
     T* sC = reinterpret_cast<T*>(smem_raw + SM::key_bytes);
     float* sF = reinterpret_cast<float*>(smem_raw + SM::bytes);  // HASF only
     __shared__ uint64_t bar;
-    __shared__ unsigned int s_tile;
+    // this tile and the next one: one thread takes the next from the dispenser and copies its split
+    // points while the block works on this one, so neither latency is waited for (669 to 651 us a
+    // layer at 2^25 terms)
+    __shared__ MergeTile s_next[2];
+    __shared__ uint32_t s_tie;
     __shared__ unsigned int s_warp[kBlock / 32];
     __shared__ unsigned int s_si[kBlock + 1], s_sj[kBlock + 1];
     __shared__ unsigned long long s_outoff;
@@ -674,14 +707,33 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
     // a slotted output's span, for the TopN pass that reads it without the host knowing m
     if (slot_count && blockIdx.x == 0 && tid == 0) ctl->span = (unsigned long long)num_tiles * (SM::TILE + 2);
     uint32_t phase = 0;  // completed phases of `bar`
+    if constexpr (CUT) {  // the last tie's rank among the rows in its place
+        if (tid == 0) {
+            const uint32_t e = CI.live.last_tie;
+            s_tie = e == kCutAllTies ? kCutAllTies : CI.pr[e / CI.slot_rows] + e % CI.slot_rows;
+        }
+    }
     // Persistent: each block takes tiles from the dispenser until none is left (the grid is
     // sized by residency, not by the tile count, which only the device knows).
-    for (;;) {
-        if (tid == 0) s_tile = atomicAdd(&ctl->tile_counter[3], 1u);
-        __syncthreads();  // also: every thread is done with the previous tile's shared memory
-        const unsigned int tile = s_tile;
+    auto copy_tile = [&](MergeTile& q, unsigned int t) {  // asynchronous (cp_async_wait_all)
+        q.tile = t;
+        if (t < num_tiles) {
+            cp_async<16>(&q.b0, bounds + t);
+            cp_async<16>(&q.b1, bounds + t + 1);
+            if constexpr (CUT) cp_async<16>(&q.slot, CI.bslot + t);
+        }
+    };
+    constexpr int kFetcher = kBlock - 1;
+    unsigned int at = 0, next_tile = 0;
+    if (tid == kFetcher) {
+        copy_tile(s_next[0], atomicAdd(&ctl->tile_counter[3], 1u));
+        cp_async_wait_all();
+    }
+    for (;; at ^= 1u) {
+        __syncthreads();  // the tile is fetched, and every thread is done with the previous one's shared memory
+        const unsigned int tile = s_next[at].tile;
         if (tile >= num_tiles) break;
-        const ulonglong2 b0 = bounds[tile], b1 = bounds[tile + 1];
+        const ulonglong2 b0 = s_next[at].b0, b1 = s_next[at].b1;
         if (!PS_GUARD(ctl, b1.x >= b0.x && b1.y >= b0.y && b1.x - b0.x + b1.y - b0.y <= (uint64_t)SM::TILE + 2 &&
                                b1.x <= n && b1.y <= m,
                       301))
@@ -689,7 +741,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
         const uint32_t cs = (uint32_t)(b1.x - b0.x), cp = (uint32_t)(b1.y - b0.y);
         // stage the two input runs: keys packed (S then P), coefficients from 16-byte aligned windows
         const uint64_t sa = b0.x & ~(uint64_t)(SM::PAD - 1), pa = b0.y & ~(uint64_t)(SM::PAD - 1);
-        const uint32_t s_off = (uint32_t)(b0.x - sa), p_off = (uint32_t)(b0.y - pa);
+        const uint32_t s_off = CUT ? 0u : (uint32_t)(b0.x - sa), p_off = (uint32_t)(b0.y - pa);
         const uint32_t sc_slots = (s_off + cs + SM::PAD - 1) / SM::PAD * SM::PAD;
         T* sSc = sC;             // S coefficient of local i at sSc[s_off + i]
         T* sPc = sC + sc_slots;  // P coefficient of local j at sPc[p_off + j]
@@ -704,7 +756,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
         if (tid == 0 && cs + cp) {
             bulk_wait_read_all();  // the previous tile's bulk store has read the staged rows
             uint32_t kbS = cs * 16u * W, kbP = cp * 16u * W;
-            uint32_t cbS = cs ? round16((s_off + cs) * (uint32_t)sizeof(T)) : 0u;
+            uint32_t cbS = cs && !CUT ? round16((s_off + cs) * (uint32_t)sizeof(T)) : 0u;
             uint32_t cbP = cp ? round16((p_off + cp) * (uint32_t)sizeof(T)) : 0u;
             uint32_t fbS = 0, fbP = 0;
             if constexpr (HASF) {
@@ -712,7 +764,24 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
                 fbP = cp ? round16((fp_off + cp) * 4u) : 0u;
             }
             mbar_arrive_expect_tx(&bar, kbS + kbP + cbS + cbP + fbS + fbP);
-            if (kbS) bulk_g2s(sSk, Sk + b0.x * 2 * W, kbS, &bar);
+            if constexpr (CUT) {
+                // own keys from their slots, a copy per slot the tile's rows lie in (two, mostly)
+                uint32_t g = s_next[at].slot.x, row = (uint32_t)b0.x, left = cs, p = s_next[at].slot.y, e = s_next[at].slot.z;
+                uint64_t* to = sSk;
+                while (left) {
+                    const uint32_t take = row < e ? min(left, e - row) : 0u;
+                    if (take) bulk_g2s(to, Sk + ((uint64_t)g * CI.slot_rows + (row - p)) * 2 * W, take * 16u * W, &bar);
+                    to += (size_t)take * 2 * W;
+                    row += take;
+                    left -= take;
+                    if (left) {
+                        p = e;
+                        e = CI.pr[++g + 1];
+                    }
+                }
+            } else {
+                if (kbS) bulk_g2s(sSk, Sk + b0.x * 2 * W, kbS, &bar);
+            }
             if (kbP) bulk_g2s(sPk, Pk + b0.y * 2 * W, kbP, &bar);
             if (cbS) bulk_g2s(sSc, Sc + sa, cbS, &bar);
             if (cbP) bulk_g2s(sPc, Pc + pa, cbP, &bar);
@@ -720,6 +789,20 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
                 if (fbS) bulk_g2s(sSf, Sf + fsa, fbS, &bar);
                 if (fbP) bulk_g2s(sPf, Pf + fpa, fbP, &bar);
             }
+        }
+        if constexpr (CUT) {
+            // own coefficients element by element (in its slot a row has any alignment)
+            const uint32_t g0 = s_next[at].slot.x, p0 = s_next[at].slot.y, e0 = s_next[at].slot.z;
+            for (uint32_t i = tid; i < cs; i += kBlock) {
+                const uint32_t row = (uint32_t)b0.x + i;
+                uint32_t g = g0, p = p0, e = e0;
+                while (row >= e) {  // row < n, the last slot's end
+                    p = e;
+                    e = CI.pr[++g + 1];
+                }
+                cp_async<(int)sizeof(T)>(sSc + i, Sc + (uint64_t)g * CI.slot_rows + (row - p));
+            }
+            cp_async_wait_all();
         }
         if (cs + cp) {  // block-uniform
             const bool ok = mbar_wait(&bar, phase & 1u, ctl, 302);
@@ -731,6 +814,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
             }
             ++phase;
         }
+        if (tid == kFetcher) next_tile = atomicAdd(&ctl->tile_counter[3], 1u);  // used after the search below
         const T* Sc_l = sSc + s_off;
         const T* Pc_l = sPc + p_off;
 
@@ -755,6 +839,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
             }
         }
         __syncthreads();
+        if (tid == kFetcher) copy_tile(s_next[at ^ 1u], next_tile);
         const uint32_t i0 = s_si[tid], j0 = s_sj[tid];
         const uint32_t ie = max(s_si[tid + 1], i0), je = max(s_sj[tid + 1], j0);
         constexpr int STEPS = ITEMS + 1;
@@ -762,8 +847,9 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
         T ov[STEPS];
         float of[STEPS];
         uint32_t i = i0, j = j0;
-        const uint32_t mask = merge_walk<W, T, STEPS, NOISE, HASF>(sSk, Sc_l, sPk, Pc_l, i, ie, j, je, L, A, keep, ok,
-                                                                  ov, NS, s_drop, sSf + fs_off, sPf + fp_off, of);
+        const uint32_t mask = merge_walk<W, T, STEPS, NOISE, HASF, CUT>(sSk, Sc_l, sPk, Pc_l, i, ie, j, je, L, A, keep,
+                                                                       ok, ov, NS, s_drop, sSf + fs_off, sPf + fp_off,
+                                                                       of, CI, s_tie, (uint32_t)b0.x);
         PS_GUARD(ctl, i >= ie && j >= je, 305);
         unsigned int total;
         const unsigned int excl = block_exclusive_sum<kBlock>(__popc(mask), s_warp, total);
@@ -818,7 +904,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
             if constexpr (NEXTF) {
                 uint64_t k[2 * W];
                 ld_row<W>(sK, q, k);
-                NX.flags[off + q] = emits_partner_regs<W, T>(NX.L, NA, k) ? 1 : 0;
+                NX.flags[(uint64_t)tile * flag_stride(SM::TILE + 2) + q] = emits_partner_regs<W, T>(NX.L, NA, k) ? 1 : 0;
             }
             float fv = 0.0f;
             if constexpr (HASF) {
@@ -827,7 +913,9 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
             }
             if (topn_hist) {
                 uint32_t bin;
-                if (hist_mode == 1)
+                if (NEXTF && hist_mode == 5)
+                    bin = cut_bin<T>(v, (uint32_t)hist_base);
+                else if (hist_mode == 1)
                     bin = octave_bin<T>(v);
                 else if (hist_mode == 2)
                     bin = (uint32_t)(window_key(mag_key<T>(v), hist_base) >> 48);
@@ -840,6 +928,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
                 atomicAdd(&s_hist[bin], 1u);
             }
         }
+        if (tid == kFetcher) cp_async_wait_all();
     }
     if (topn_hist) {
         __syncthreads();
@@ -852,6 +941,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 4 : 1) k_merge(const uint64_t
             if (s_drop[q]) atomicAdd(&noise_drops[q], (unsigned long long)s_drop[q]);
     }
     if (tid == 0) bulk_wait_read_all();  // shared memory stays valid until the last copy has read it
+    if (tid == kFetcher) cp_async_wait_all();
 }
 
 // One launch resets what a rotation layer's kernels count on: the partner count (unless the
@@ -893,7 +983,7 @@ cudaError_t launch_rotation_layer(const RotationArgs<W, T>& a, cudaStream_t st) 
     constexpr int MT = RotTile<W>::kMergeTile;
     Ctl* ctl = a.ctl;
     cudaError_t e;
-    const uint64_t m_hi = a.L.partners ? a.n : 0;  // partners cannot outnumber the terms
+    const uint64_t m_hi = a.cut ? a.cut_m : a.L.partners ? a.n : 0;  // partners cannot outnumber the terms
     if (m_hi > a.p_cap) return cudaErrorMemoryAllocation;  // caller sized the partner buffers by n
     // look-back words: the classify's tiles first, then the merge's (when it is not slotted)
     const uint32_t ctiles = m_hi > 0 ? (uint32_t)((a.n + CT - 1) / CT) : 0u;
@@ -906,7 +996,17 @@ cudaError_t launch_rotation_layer(const RotationArgs<W, T>& a, cudaStream_t st) 
                                              a.noise ? a.noise_drops : nullptr, a.preclassified);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if (m_hi > 0) {
+    CutLive live{};
+    if (a.cut) {
+        // |c|^2 as the select keys order it: key - 1 is its bit pattern
+        const unsigned long long bits = a.cut_boundary - 1;
+        std::memcpy(&live.bound, &bits, sizeof bits);
+        live.last_tie = a.cut_last_tie;
+        // 1-3. the cut before this layer listed its partners and scanned their levels
+        if ((e = CutOps<W, T>::place(*a.cut, a.L, a.cut_tiles, live, a.cut_m, a.Pk, a.Pc, a.cut_pr, a.sms, st,
+                                     a.prof)) != cudaSuccess)
+            return e;
+    } else if (m_hi > 0) {
         // 1. classify (unless the TopN compaction before this layer listed the partners)
         if (!a.preclassified) {
             const uint32_t tiles = ctiles;
@@ -982,7 +1082,12 @@ cudaError_t launch_rotation_layer(const RotationArgs<W, T>& a, cudaStream_t st) 
         return cudaSuccess;
     }
     if ((a.slot_count ? (uint64_t)mtiles_hi * (MT + 2) : total_hi) > a.out_cap) return cudaErrorMemoryAllocation;
-    {
+    if (a.cut) {
+        const CutStore S{a.cut_pr, a.cut_tiles, a.cut->slot_rows};
+        if ((e = CutOps<W, T>::partition(a.Sk, a.n, S, a.Pk, a.cut_m, (uint32_t)MT, a.bounds, a.cut_bslot, a.sms, st,
+                                         a.prof)) != cudaSuccess)
+            return e;
+    } else {
         uint32_t warps = mtiles_hi + 1;
         uint32_t blocks = std::min<uint32_t>((warps + 7) / 8, 8u * (uint32_t)(a.sms > 0 ? a.sms : 1));
         a.prof->begin(K_PARTITION, 0.0, st);
@@ -994,10 +1099,34 @@ cudaError_t launch_rotation_layer(const RotationArgs<W, T>& a, cudaStream_t st) 
     // injection the dispenser starts at tile 1, so tile 0 never publishes and tile 1's bounded
     // look-back gives up)
     const size_t smem = MergeSmem<W, T>::bytes;
-    static std::atomic<int> merge_per_sm[4];
+    static std::atomic<int> merge_per_sm[6];
     const long long stall = a.inject_stall ? (long long)a.stall_limit : 0ll;
     a.prof->begin(K_MERGE, 0.0, st);
-    if (a.noise) {
+    if (a.cut) {
+        CutIn ci;
+        ci.pr = a.cut_pr;
+        ci.bslot = a.cut_bslot;
+        ci.slot_rows = a.cut->slot_rows;
+        ci.live = live;
+        if (a.next_flags) {
+            const int mper = resident_blocks(k_merge<W, T, false, false, true, true>, kBlock, smem, merge_per_sm[4]);
+            const uint32_t mgrid = (uint32_t)std::min<uint64_t>(mtiles_hi, (uint64_t)mper * (a.sms > 0 ? a.sms : 1));
+            NextFlagArg<W> nx;
+            nx.L = a.next_L;
+            nx.flags = a.next_flags;
+            k_merge<W, T, false, false, true, true><<<mgrid, kBlock, smem, st>>>(
+                a.Sk, a.Sc, a.n, a.Pk, a.Pc, a.bounds, a.L, a.keep, a.Ok, a.Oc, a.out_cap, merge_status, ctl,
+                a.topn_hist, a.topn_hist_mode, a.topn_hist_base, a.slot_count, stall, NoNoise{},
+                nullptr, nullptr, nullptr, nullptr, nx, ci);
+        } else {
+            const int mper = resident_blocks(k_merge<W, T, false, false, false, true>, kBlock, smem, merge_per_sm[5]);
+            const uint32_t mgrid = (uint32_t)std::min<uint64_t>(mtiles_hi, (uint64_t)mper * (a.sms > 0 ? a.sms : 1));
+            k_merge<W, T, false, false, false, true><<<mgrid, kBlock, smem, st>>>(
+                a.Sk, a.Sc, a.n, a.Pk, a.Pc, a.bounds, a.L, a.keep, a.Ok, a.Oc, a.out_cap, merge_status, ctl,
+                a.topn_hist, a.topn_hist_mode, a.topn_hist_base, a.slot_count, stall, NoNoise{},
+                nullptr, nullptr, nullptr, nullptr, NoNextFlag{}, ci);
+        }
+    } else if (a.noise) {
         const int mper = resident_blocks(k_merge<W, T, true, false>, kBlock, smem, merge_per_sm[1]);
         const uint32_t mgrid = (uint32_t)std::min<uint64_t>(mtiles_hi, (uint64_t)mper * (a.sms > 0 ? a.sms : 1));
         k_merge<W, T, true, false><<<mgrid, kBlock, smem, st>>>(
@@ -1099,8 +1228,11 @@ template uint64_t merge_span_rows<4>(uint64_t);
 template <int W, typename T>
 cudaError_t configure_rotation_kernels() {
     cudaError_t e = cudaSuccess;
-    const void* kernels[4] = {(const void*)k_merge<W, T, false, false>, (const void*)k_merge<W, T, true, false>,
-                              (const void*)k_merge<W, T, false, true>, (const void*)k_merge<W, T, false, false, true>};
+    const void* kernels[6] = {(const void*)k_merge<W, T, false, false>, (const void*)k_merge<W, T, true, false>,
+                              (const void*)k_merge<W, T, false, true>, (const void*)k_merge<W, T, false, false, true>,
+                              (const void*)k_merge<W, T, false, false, true, true>,
+                              (const void*)k_merge<W, T, false, false, false, true>};
+    e = CutOps<W, T>::configure();
     for (const void* k : kernels) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -48,6 +48,10 @@ struct SlotWalk {
     }
     // call only for a row below the store's span
     __device__ bool live(const SlotMap& s) const { return !s.count || r < __ldg(s.count + q); }
+    // its partner test among the tile's flag_stride bytes (a slotted store's row)
+    __device__ bool flag(const SlotMap& s, const uint8_t* __restrict__ f) const {
+        return f[(uint64_t)q * flag_stride(s.rows) + r] != 0;
+    }
     __device__ void step32(const SlotMap& s) {
         r += 32;
         if (r >= s.rows) {
@@ -1073,8 +1077,8 @@ __global__ void __launch_bounds__(kThreads) k_topn_compact(const uint64_t* __res
 // the first of a warp, which k_level_reduce resolves), and the last tile publishes the partner
 // count in count[0], as k_classify does.  Otherwise (the quota cuts the ties, or the boundary is
 // NaN) the plain compaction runs and aux[7] tells the host that the next layer classifies itself.
-// FLAGS: the layer's merge wrote each row's partner test under the next layer (nflag, one byte
-// per row of the slotted store), so the first pass reads a byte instead of the key.
+// FLAGS: the layer's merge wrote each row's partner test under the next layer (nflag, a byte per
+// row of the slotted store), so the first pass reads no key.
 // SCORE: the inherited learned pass (keys score_key(c, f) from the carried predictions fin,
 // which the kept rows carry to fout).
 template <int W, typename T, bool FLAGS, bool SCORE = false>
@@ -1133,7 +1137,7 @@ __global__ void __launch_bounds__(kThreads, W == 1 ? (SCORE ? 4 : 8) : (W == 2 ?
             else
                 mk = mag_key<T>(coef[e]);
             if constexpr (FLAGS) {
-                const bool f = nflag[e] != 0;
+                const bool f = sw.flag(slots, nflag);
                 if (sw.live(slots) && mk >= boundary) {
                     kept = true;
                     part = f;
@@ -1718,24 +1722,29 @@ cudaError_t StoreOps<W, T>::topn(const uint64_t* keys, const T* coef, uint64_t n
 template <int W, typename T>
 cudaError_t StoreOps<W, T>::densify(const uint64_t* keys, const T* coef, uint64_t n, SlotMap slots, uint64_t* okeys,
                                     T* ocoef, unsigned long long* status, Ctl* ctl, unsigned long long* host_count,
-                                    uint64_t* out_n, cudaStream_t st, KernelProf* prof, const float* fin, float* fout) {
+                                    uint64_t* out_n, cudaStream_t st, KernelProf* prof, const float* fin, float* fout,
+                                    unsigned long long boundary, unsigned long long above,
+                                    unsigned long long keep_n) {
     if (n == 0) {
         *out_n = 0;
         return cudaSuccess;
     }
     unsigned long long* init = host_count + 8;
-    for (int q = 0; q < 4; ++q) init[q] = 0ull;  // no boundary, no quota
-    cudaMemcpyAsync(ctl->aux, init, 4 * sizeof(unsigned long long), cudaMemcpyHostToDevice, st);
+    // no boundary: every live row; with one: the `above` rows above it and the first keep_n - above
+    // equal to it
+    for (int q = 0; q < 6; ++q) init[q] = q == 0 ? boundary : q == 3 ? above : 0ull;
+    const int mode = boundary ? 0 : 3;
+    cudaMemcpyAsync(ctl->aux, init, 6 * sizeof(unsigned long long), cudaMemcpyHostToDevice, st);
     const uint32_t tiles = (uint32_t)((n + kThreads * 16 - 1) / (kThreads * 16));
     cudaMemsetAsync(status, 0, (size_t)tiles * sizeof(unsigned long long), st);
     cudaMemsetAsync(&ctl->tile_counter[6], 0, sizeof(unsigned int), st);
     prof->begin(K_TOPN_COMPACT, 0.0, st);
     if (fout)
-        k_topn_compact<W, T, true><<<tiles, kThreads, 0, st>>>(keys, coef, nullptr, 3, 0ull, n, 0ull, okeys, ocoef,
-                                                               status, ctl, slots, fin, fout, 0);
+        k_topn_compact<W, T, true><<<tiles, kThreads, 0, st>>>(keys, coef, nullptr, mode, 0ull, n, keep_n, okeys,
+                                                               ocoef, status, ctl, slots, fin, fout, 0);
     else
-        k_topn_compact<W, T, false><<<tiles, kThreads, 0, st>>>(keys, coef, nullptr, 3, 0ull, n, 0ull, okeys, ocoef,
-                                                                status, ctl, slots, nullptr, nullptr, 0);
+        k_topn_compact<W, T, false><<<tiles, kThreads, 0, st>>>(keys, coef, nullptr, mode, 0ull, n, keep_n, okeys,
+                                                                ocoef, status, ctl, slots, nullptr, nullptr, 0);
     prof->end(st);
     cudaError_t e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

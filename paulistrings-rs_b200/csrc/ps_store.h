@@ -98,11 +98,13 @@ struct StoreOps {
     // Can topn run deferred (the whole select in one cooperative launch on this device)?
     static bool cooperative_select();
     // Compact the live rows of a slotted store of n rows (its span) into okeys / ocoef, in order;
-    // *out_n = rows kept.  Reads the counts and error words into host_count (synchronizes).
+    // *out_n = rows kept.  boundary > 0: only the `above` rows with a larger select key and
+    // the first keep_n - above equal to it.  Reads the counts and error words into host_count (synchronizes).
     static cudaError_t densify(const uint64_t* keys, const T* coef, uint64_t n, SlotMap slots, uint64_t* okeys,
                                T* ocoef, unsigned long long* status, Ctl* ctl, unsigned long long* host_count,
                                uint64_t* out_n, cudaStream_t st, KernelProf* prof, const float* fin = nullptr,
-                               float* fout = nullptr);
+                               float* fout = nullptr, unsigned long long boundary = 0,
+                               unsigned long long above = 0, unsigned long long keep_n = 0);
     // ApproxTopN (crates/paulistrings/src/truncation/builtin.rs:240-468): every octave of |c|^2
     // above the boundary octave kept, then the first quota boundary terms in key order.
     // hist: 2048 words, zero on entry and exit, holding the octave histogram when hist_ready;
