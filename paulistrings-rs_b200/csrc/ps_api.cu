@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/paulistrings_b200.h"
@@ -98,6 +99,7 @@ struct ps_sum {
     Buf sort_status;
     Buf up_x, up_z, up_c, up_k, up_v0, up_v1, up_c0, up_st;  // ingest / readout staging, grow-only
     LevelList* levels = nullptr;  // host scratch
+    std::vector<ps_table> tables; // a propagation's prepared channels
     KernelProf prof;
     // Light-cone skip: `support` holds a superset of the qubits any term touches (exact after an
     // upload, widened by each layer's support), and keep_clean says every term already passed
@@ -184,9 +186,54 @@ ps_status cuda_fail(ps_sum* s, cudaError_t e, const char* where) {
     return set_err(s, st, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
-// Grow-only buffer; contents are not preserved.  A buffer that must grow grows by half again
-// at least (exactly to the request when that much does not fit), so a sum that grows a little
-// every layer does not free and allocate -- two device-wide synchronizations -- every layer.
+// Scratch memory of the handles comes from one stream-ordered pool per device (the driver's, so
+// handles on any threads and streams share it safely): a handle made for one call, and a buffer
+// that grows, take memory that an earlier handle gave back instead of mapping new pages and
+// synchronizing the device (most of a 16-site quench from host arrays was its two handles' allocations:
+// 12-24 ms a call before, 8-13 with the pool).  At most kPoolKeep bytes stay mapped while no handle uses them; the rest
+// goes back to the device at the next synchronization, and all of it when an allocation fails.
+constexpr uint64_t kPoolKeep = 256ull << 20;
+cudaMemPool_t device_pool(int dev) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    static bool tried[64] = {};
+    if (dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!tried[dev]) {
+        tried[dev] = true;
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof props);
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            pools[dev] = nullptr;
+        }
+    }
+    return pools[dev];
+}
+
+// bytes on the current device, usable in `st`'s order (any order once `st` was synchronized).
+cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t st) {
+    int dev = -1;
+    cudaMemPool_t pool = cudaGetDevice(&dev) == cudaSuccess ? device_pool(dev) : nullptr;
+    if (!pool) return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaStreamSynchronize(st);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    return e;
+}
+
+// The store's own columns, and a scorer's buffers, which the streams of the sums it is attached to
+// read too: plain allocations.  Growth as below.
 cudaError_t ensure(Buf& b, size_t bytes) {
     if (b.bytes >= bytes && b.p) return cudaSuccess;
     size_t cap = b.p && b.bytes ? std::max(bytes, b.bytes + b.bytes / 2) : bytes;
@@ -206,6 +253,33 @@ cudaError_t ensure(Buf& b, size_t bytes) {
     b.bytes = cap;
     return cudaSuccess;
 }
+void release(Buf& b) {
+    if (b.p) cudaFree(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+}
+
+// Grow-only buffer of one stream; contents are not preserved.  A buffer that must grow grows by half
+// again at least (exactly to the request when that much does not fit).
+cudaError_t ensure(Buf& b, size_t bytes, cudaStream_t st) {
+    if (b.bytes >= bytes && b.p) return cudaSuccess;
+    size_t cap = b.p && b.bytes ? std::max(bytes, b.bytes + b.bytes / 2) : bytes;
+    if (b.p) cudaFreeAsync(b.p, st);  // after the work queued on it
+    b.p = nullptr;
+    b.bytes = 0;
+    cudaError_t e = device_alloc(&b.p, cap + kPad, st);
+    if (e == cudaErrorMemoryAllocation && cap > bytes) {
+        cudaGetLastError();
+        cap = bytes;
+        e = device_alloc(&b.p, cap + kPad, st);
+    }
+    if (e != cudaSuccess) {
+        b.p = nullptr;
+        return e;
+    }
+    b.bytes = cap;
+    return cudaSuccess;
+}
 
 // ensure() through the handle, so an injected allocation failure can take its place.
 cudaError_t ensure(ps_sum* s, Buf& b, size_t bytes) {
@@ -214,11 +288,13 @@ cudaError_t ensure(ps_sum* s, Buf& b, size_t bytes) {
         if (s->fault_oom_after == 0) return cudaErrorMemoryAllocation;  // until disarmed
         --s->fault_oom_after;
     }
-    return ensure(b, bytes);
+    const bool column = &b == &s->keys[0] || &b == &s->keys[1] || &b == &s->coef[0] || &b == &s->coef[1] ||
+                        &b == &s->fcol[0] || &b == &s->fcol[1];
+    return column ? ensure(b, bytes) : ensure(b, bytes, s->stream);
 }
 
-void release(Buf& b) {
-    if (b.p) cudaFree(b.p);
+void release(Buf& b, cudaStream_t st) {
+    if (b.p) cudaFreeAsync(b.p, st);
     b.p = nullptr;
     b.bytes = 0;
 }
@@ -355,22 +431,6 @@ struct HostKey {
     uint64_t x[PS_MAX_W], z[PS_MAX_W];
 };
 
-bool host_anticommutes(const HostKey& a, const uint64_t* gx, const uint64_t* gz, int W) {
-    uint64_t f = 0;
-    for (int i = 0; i < W; ++i) f ^= (a.x[i] & gz[i]) ^ (a.z[i] & gx[i]);
-    return (__builtin_popcountll(f) & 1) != 0;
-}
-
-unsigned host_phase(const HostKey& k, const uint64_t* gx, const uint64_t* gz, int W) {
-    unsigned d = 0;
-    for (int i = 0; i < W; ++i) {
-        uint64_t a = k.x[i], b = k.z[i], c = gx[i], e = gz[i];
-        d += 2u * __builtin_popcountll(b & c) + __builtin_popcountll(a & b) + __builtin_popcountll(c & e) -
-             __builtin_popcountll((a ^ c) & (b ^ e));
-    }
-    return d & 3u;
-}
-
 HostKey lift_local(const ps_table& t, unsigned d) {
     HostKey k;
     std::memset(&k, 0, sizeof k);
@@ -380,16 +440,6 @@ HostKey lift_local(const ps_table& t, unsigned d) {
         if ((d >> (2 * j + 1)) & 1u) k.z[q / 64] |= 1ull << (q % 64);
     }
     return k;
-}
-
-unsigned local_bits(const ps_table& t, const HostKey& k) {
-    unsigned s = 0;
-    for (int j = 0; j < t.k; ++j) {
-        uint32_t q = t.qubits[j];
-        s |= (unsigned)((k.x[q / 64] >> (q % 64)) & 1u) << (2 * j);
-        s |= (unsigned)((k.z[q / 64] >> (q % 64)) & 1u) << (2 * j + 1);
-    }
-    return s;
 }
 
 void push_deltas(ps_table& t, const double (&table)[16][16], int W) {
@@ -609,13 +659,20 @@ bool named_ptm(const ps_channel* ch, int& k, double (&ptm)[16][16], std::string&
     }
 }
 
-ps_status build_table(int nq, const ps_channel* ch, int adjoint, ps_table* out, std::string& why) {
+// whole: the entries past num_entries zero too (a table that leaves the library).
+ps_status build_table(int nq, const ps_channel* ch, int adjoint, ps_table* out, std::string& why, bool whole = false) {
     const int W = width_for(nq);
     if (!W) {
         why = "num_qubits out of range";
         return PS_ERR_INVALID;
     }
-    std::memset(out, 0, sizeof *out);
+    if (whole) std::memset(out, 0, sizeof *out);
+    out->mode = out->k = 0;
+    out->qubits[0] = out->qubits[1] = 0;
+    out->num_entries = 0;
+    std::memset(out->gen_x, 0, sizeof out->gen_x);
+    std::memset(out->gen_z, 0, sizeof out->gen_z);
+    out->cos_theta = out->sin_theta = 0.0;
     out->width = W;
     if (!ch || ch->num_support < 0 || ch->num_support > 64 * PS_MAX_W || (ch->num_support && !ch->qubits)) {
         why = "channel: bad support";
@@ -681,25 +738,50 @@ ps_status build_table(int nq, const ps_channel* ch, int adjoint, ps_table* out, 
             }
         }
         out->k = k;
-        double table[16][16];
-        std::memset(table, 0, sizeof table);
-        int dim = 1 << (2 * k);
-        for (int s = 0; s < dim; ++s) {
-            HostKey in = lift_local(*out, (unsigned)s);
-            if (!host_anticommutes(in, gx, gz, W)) {
-                table[s][s] += 1.0;
-                continue;
-            }
-            table[s][s] += 1.0 * cs;
-            unsigned total = (1u + host_phase(in, gx, gz, W)) & 3u;
-            HostKey o = in;
-            for (int w = 0; w < W; ++w) {
-                o.x[w] ^= gx[w];
-                o.z[w] ^= gz[w];
-            }
-            table[s][local_bits(*out, o)] += ((total & 2u) ? -1.0 : 1.0) * sn;
+        // c -> c for a pattern that commutes with the generator, c cos and its partner +-c sin otherwise
+        // (mul_assign's phase, 2bc + ab + cd - (a^c)(b^d), on the support's bits); an entry exists when it reaches
+        // any pattern
+        unsigned g = 0;
+        for (int j = 0; j < k; ++j) {
+            const uint32_t q = out->qubits[j];
+            g |= (unsigned)((gx[q / 64] >> (q % 64)) & 1u) << (2 * j) | (unsigned)((gz[q / 64] >> (q % 64)) & 1u) << (2 * j + 1);
         }
-        push_deltas(*out, table, W);
+        const int dim = 1 << (2 * k);
+        double own[16] = {0.0}, part[16] = {0.0};
+        bool has_own = false, has_part = false;
+        for (int s = 0; s < dim; ++s) {
+            unsigned anti = 0, phase = 0;
+            for (int j = 0; j < k; ++j) {
+                const unsigned a = (s >> (2 * j)) & 1u, b = (s >> (2 * j + 1)) & 1u;
+                const unsigned c = (g >> (2 * j)) & 1u, d = (g >> (2 * j + 1)) & 1u;
+                anti ^= (a & d) ^ (b & c);
+                phase += 2u * (b & c) + (a & b) + (c & d) - ((a ^ c) & (b ^ d));
+            }
+            if (!anti) {
+                own[s] = 1.0;
+            } else {
+                own[s] = 0.0 + cs;
+                part[s] = 0.0 + (((1u + phase) & 2u) ? -1.0 : 1.0) * sn;
+            }
+            has_own = has_own || own[s] != 0.0;
+            has_part = has_part || part[s] != 0.0;
+        }
+        if (g == 0) {  // the identity: a table of one entry
+            for (int s = 0; s < dim; ++s) part[s] = 0.0;
+            has_part = false;
+        }
+        for (int e = 0; e < 2; ++e) {
+            if (!(e ? has_part : has_own)) continue;
+            ps_table_entry& t = out->entries[out->num_entries++];
+            std::memset(&t, 0, sizeof t);
+            t.local_delta = e ? g : 0u;
+            if (e)
+                for (int w = 0; w < W; ++w) {
+                    t.mask_x[w] = gx[w];
+                    t.mask_z[w] = gz[w];
+                }
+            for (int s = 0; s < dim; ++s) t.amplitude[s] = e ? part[s] : own[s];
+        }
         return PS_OK;
     }
     if (ch->kind == PS_CH_DEPOLARIZING) {
@@ -1467,7 +1549,7 @@ struct Engine {
     // partner bits, any keep program and at most one plain TopN pass; layers the light-cone skip
     // passes over and folded noise are resolved here as the per-layer path resolves them.  It is not used while per-kernel profiling or a
     // failure injection is on (both act on the per-layer kernels).
-    static ps_status run_layers(ps_sum* s, const std::vector<ps_table>& tables, uint64_t li, const ps_policy* policy,
+    static ps_status run_layers(ps_sum* s, const ps_table* tables, uint64_t ntables, uint64_t li, const ps_policy* policy,
                                 uint64_t* terms_after, ps_run_stats* rs, uint64_t* consumed) {
         *consumed = 0;
         if (s->prof.events || s->fault_oom_after >= 0 || s->fault_stall || s->fault_flag) return PS_OK;
@@ -1506,9 +1588,26 @@ struct Engine {
         uint64_t sup[W];
         for (int w = 0; w < W; ++w) sup[w] = s->support[w];
         bool clean = s->support_known && s->keep_clean && std::memcmp(&keep, &s->clean_keep, sizeof keep) == 0;
-        const uint64_t end = std::min<uint64_t>(tables.size(), li + kRunMaxLayers);
+        const uint64_t end = std::min<uint64_t>(ntables, li + kRunMaxLayers);
         uint64_t grow = n0;  // bound on the rows of the run
         for (uint64_t c = li; c < end;) {
+            // passed over by the light-cone skip (a rotation's table, before its device form is built)
+            if (clean && tables[c].mode == PS_TABLE_LOCAL && tables[c].num_entries == 2 &&
+                tables[c].entries[0].local_delta == 0 && (T)tables[c].entries[0].amplitude[0] == T(1) &&
+                (T)tables[c].entries[1].amplitude[0] == T(0)) {
+                Entry en{};
+                table_support<W>(tables[c], en.lsup);
+                bool skip = true;
+                for (int w = 0; w < W; ++w) skip = skip && !(en.lsup[w] & sup[w]);
+                if (skip) {
+                    en.channels = 1;
+                    en.prog = -1;
+                    en.partners = true;
+                    entries.push_back(en);
+                    ++c;
+                    continue;
+                }
+            }
             uint64_t fj = c;
             while (fj < end && fj - c < (uint64_t)kMaxNoise && foldable_noise(tables[fj], s->nq)) ++fj;
             Entry en{};
@@ -1525,7 +1624,7 @@ struct Engine {
                 if (to_rot_layer<W, T>(tables[c], R, *s->levels, why, &general) != PS_OK || general) break;
                 if (R.partners && s->levels->n > kRunLevels) break;
                 // noise cut off from its rotation by the end of the run is left to the next one
-                if (fj > c && fj == end && end < tables.size()) break;
+                if (fj > c && fj == end && end < ntables) break;
             }
             table_support<W>(tables[at], en.lsup);
             en.channels = at - c + 1;
@@ -2418,7 +2517,7 @@ ps_status ps_create(int32_t device, int32_t num_qubits, int32_t dtype, ps_sum** 
     if (e == cudaSuccess) e = cudaMalloc(&s->sort.base, 16 * W * 256 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost(&s->sort.host_hist, 16 * W * 256 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost(&s->sort.host_base, 16 * W * 256 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = ensure(s->hist, kTopnBinsN * sizeof(unsigned int));
+    if (e == cudaSuccess) e = ensure(s->hist, kTopnBinsN * sizeof(unsigned int), s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->hist.p, 0, kTopnBinsN * sizeof(unsigned int), s->stream);
     if (e == cudaSuccess) {
         ps_status st = dispatch<Engine>(s, [&](auto op) {
@@ -2443,16 +2542,17 @@ ps_status ps_destroy(ps_sum* s) {
     if (!s) return PS_OK;
     DeviceGuard g(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (Buf* b : {&s->fcol[0], &s->fcol[1], &s->pf, &s->run_prog, &s->run_state, &s->run_sums})
-        release(*b);
+    for (Buf* b : {&s->fcol[0], &s->fcol[1], &s->keys[0], &s->keys[1], &s->coef[0], &s->coef[1]}) release(*b);
+    for (Buf* b : {&s->pf, &s->run_prog, &s->run_state, &s->run_sums})
+        release(*b, s->stream);
     if (s->hrun) cudaFreeHost(s->hrun);
-    for (Buf* b : {&s->keys[0], &s->keys[1], &s->coef[0], &s->coef[1], &s->pk, &s->pc, &s->idx, &s->dv, &s->fv,
+    for (Buf* b : {&s->pk, &s->pc, &s->idx, &s->dv, &s->fv,
                    &s->slots, &s->status, &s->bounds, &s->hist, &s->cand, &s->partial, &s->dout, &s->sort_status,
                    &s->up_x, &s->up_z, &s->up_c, &s->up_k, &s->up_v0, &s->up_v1, &s->up_c0, &s->up_st, &s->sel,
                    &s->cnorms, &s->cfirst, &s->slot_count[0], &s->slot_count[1], &s->noise_drops, &s->nflag,
                    &s->cut_tiles, &s->cut_blocks, &s->cut_plist, &s->cut_D, &s->cut_cand, &s->cut_state, &s->cut_pr,
                    &s->cut_bslot})
-        release(*b);
+        release(*b, s->stream);
     if (s->ctl) cudaFree(s->ctl);
     if (s->sort.hist) cudaFree(s->sort.hist);
     if (s->sort.base) cudaFree(s->sort.base);
@@ -2500,7 +2600,7 @@ ps_status ps_prepare_channel(int32_t num_qubits, int32_t dtype, const ps_channel
     (void)dtype;
     if (!out || !channel) return PS_ERR_INVALID;
     std::string why;
-    return build_table(num_qubits, channel, adjoint, out, why);
+    return build_table(num_qubits, channel, adjoint, out, why, true);
 }
 
 ps_status ps_apply_layer(ps_sum* s, const ps_table* table, const ps_policy* policy, ps_layer_stats* stats) {
@@ -2532,7 +2632,8 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
     const bool adjoint = direction == PS_HEISENBERG;
     // Every channel is prepared before the first layer, so a bad channel fails the call
     // with the input untouched.
-    std::vector<ps_table> tables(num_channels);
+    std::vector<ps_table>& tables = s->tables;  // kept by the handle: 6 KB each, written as far as used
+    if (tables.size() < num_channels) tables.resize(num_channels);
     for (uint64_t li = 0; li < num_channels; ++li) {
         uint64_t ci = adjoint ? num_channels - 1 - li : li;
         ps = build_table(s->nq, &channels[ci], adjoint ? 1 : 0, &tables[li], why);
@@ -2553,7 +2654,7 @@ ps_status ps_propagate(ps_sum* s, const ps_channel* channels, uint64_t num_chann
     const uint64_t collapses0 = s->collapses;
     for (uint64_t li = 0; li < num_channels; ++li) {
         uint64_t ran = 0;
-        ps = dispatch<Engine>(s, [&](auto op) { return decltype(op)::run_layers(s, tables, li, policy, terms_after, &rs, &ran); });
+        ps = dispatch<Engine>(s, [&](auto op) { return decltype(op)::run_layers(s, tables.data(), num_channels, li, policy, terms_after, &rs, &ran); });
         if (ps != PS_OK) {
             s->err = "layers from " + std::to_string(li) + ": " + s->err;
             break;

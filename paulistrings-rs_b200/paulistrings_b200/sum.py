@@ -73,24 +73,26 @@ def product_basis(state: str, num_qubits: int, W: int):
         if uni in ("z+", "y+"):
             az[:] = full
         return ax, az, neg
-    table = {"0": (0, 1, 0), "1": (0, 1, 1), "+": (1, 0, 0), "-": (1, 0, 1), "r": (1, 1, 0), "l": (1, 1, 1)}
     if len(state) != num_qubits:
         raise ValueError(
             f"unknown product state {state!r}: a per-qubit label string over \"01+-rl\" needs one character "
             f"per qubit (got {len(state)}, num_qubits is {num_qubits}); the uniform names are \"x+\", \"y+\", \"z+\""
         )
-    for q, ch in enumerate(state):
-        if ch not in table:
-            raise ValueError(f"unknown product state {state!r}: {ch!r} at qubit {q} is not a per-qubit label")
-        bx, bz, bn = table[ch]
-        bit = np.uint64(1) << np.uint64(q % 64)
-        if bx:
-            ax[q // 64] |= bit
-        if bz:
-            az[q // 64] |= bit
-        if bn:
-            neg[q // 64] |= bit
+    codes = np.frombuffer(state.encode("utf-32-le"), np.uint32)
+    bits = _PRODUCT_BITS[np.minimum(codes, 255)]
+    if (bits & 8).any():
+        q = int(np.nonzero(bits & 8)[0][0])
+        raise ValueError(f"unknown product state {state!r}: {state[q]!r} at qubit {q} is not a per-qubit label")
+    for j, mask in enumerate((ax, az, neg)):
+        packed = np.packbits((bits >> j) & 1, bitorder="little")
+        mask.view(np.uint8)[: len(packed)] = packed
     return ax, az, neg
+
+
+# per character: 1 x axis, 2 z axis, 4 negative; 8 not a label
+_PRODUCT_BITS = np.full(256, 8, np.uint8)
+for _ch, _bits in {"0": 2, "1": 6, "+": 1, "-": 5, "r": 3, "l": 7}.items():
+    _PRODUCT_BITS[ord(_ch)] = _bits
 
 
 def _parse_direction(direction) -> int:
@@ -177,9 +179,9 @@ class GpuPauliSum:
         host buffers with at least ``len(self)`` rows), returning views of the filled rows."""
         n = len(self)
         if out is None:
-            x = np.zeros((n, self.W), dtype=np.uint64)
-            z = np.zeros((n, self.W), dtype=np.uint64)
-            c = np.zeros(n, dtype=np.float64)
+            x = np.empty((n, self.W), dtype=np.uint64)
+            z = np.empty((n, self.W), dtype=np.uint64)
+            c = np.empty(n, dtype=np.float64)
         else:
             x, z, c = out
             if x.shape[0] < n or z.shape[0] < n or c.shape[0] < n or x.dtype != np.uint64 or c.dtype != np.float64:
