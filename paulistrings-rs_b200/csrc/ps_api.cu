@@ -2410,7 +2410,10 @@ struct Engine {
             ps_status ps = densify(s, "expectation");
             if (ps != PS_OK) return ps;
         }
-        cudaError_t e = ensure(s, s->partial, kExpectBlocks * sizeof(double));
+        const bool fresh = !s->partial.p;
+        cudaError_t e = ensure(s, s->partial, (kExpectBlocks + 1) * sizeof(double));
+        if (e == cudaSuccess && fresh)
+            e = cudaMemsetAsync(static_cast<double*>(s->partial.p) + kExpectBlocks, 0, sizeof(double), s->stream);
         if (e == cudaSuccess) e = ensure(s, s->dout, sizeof(double));
         if (e != cudaSuccess) return cuda_fail(s, e, "expectation: scratch");
         e = StoreOps<W, T>::expectation(K(s, s->cur), C(s, s->cur), s->n, ax, az, neg, (double*)s->partial.p,

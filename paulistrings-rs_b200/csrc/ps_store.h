@@ -122,6 +122,7 @@ struct StoreOps {
                                        double* host_norms, uint64_t* first, uint64_t* host_first, uint32_t* mult,
                                        unsigned long long* status, Ctl* ctl, unsigned long long* host_count,
                                        uint64_t* out_n, bool* drawable, cudaStream_t st, KernelProf* prof);
+    // partial: kExpectBlocks + 1 doubles, the last one zero before the first call
     static cudaError_t expectation(const uint64_t* keys, const T* coef, uint64_t n, const uint64_t* ax,
                                    const uint64_t* az, const uint64_t* neg, double* partial, double* out_dev, int sms,
                                    cudaStream_t st, KernelProf* prof);
