@@ -964,6 +964,87 @@ ps_status to_rot_layer(const ps_table& t, RotLayer<W>& L, LevelList& lv, std::st
     return PS_OK;
 }
 
+// A signed permutation of the strings as steps on the partner path.  Every pattern of such a table
+// (CNOT, CZ, SWAP and their unitaries) maps to one pattern with a sign, and when the patterns that
+// move by the same delta are closed under the map (an involution), each delta is a rotation-shaped
+// step of its own: its patterns' rows move, all others stay, and no later step touches them again.
+// So the layer is at most three passes of the partner path instead of a radix sort on every key
+// byte.  undo: the step taken back (a run that fails between steps).
+template <int W>
+struct PermStep {
+    RotLayer<W> L, undo;
+    LevelList lv;
+};
+template <int W, typename T>
+bool permutation_steps(const ps_table& t, std::vector<PermStep<W>>& steps) {
+    steps.clear();
+    if (t.mode != PS_TABLE_LOCAL || t.k < 1 || t.k > 2) return false;
+    const int dim = 1 << (2 * t.k);
+    unsigned delta[16];
+    double amp[16];
+    int entry[16];
+    for (int s = 0; s < dim; ++s) {
+        int found = 0;
+        for (int e = 0; e < t.num_entries; ++e) {
+            const T a = (T)t.entries[e].amplitude[s];
+            if (a == T(0)) continue;
+            ++found;
+            delta[s] = t.entries[e].local_delta;
+            amp[s] = (double)a;
+            entry[s] = e;
+        }
+        if (found != 1 || (amp[s] != 1.0 && amp[s] != -1.0) || delta[s] >= (unsigned)dim) return false;
+    }
+    for (int s = 0; s < dim; ++s)
+        if (delta[s ^ delta[s]] != delta[s]) return false;
+    if (delta[0] != 0 || amp[0] != 1.0) return false;
+    for (unsigned g = 1; g < (unsigned)dim; ++g) {
+        int e = -1;
+        for (int s = 0; s < dim; ++s)
+            if (delta[s] == g) e = entry[s];
+        if (e < 0) continue;
+        steps.emplace_back();
+        PermStep<W>& st = steps.back();
+        RotLayer<W>& L = st.L;
+        std::memset(&L, 0, sizeof L);
+        L.wide = 2;
+        L.partners = 1;
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t q = t.qubits[j < t.k ? j : 0];
+            L.qw[j] = (int)(q / 64);
+            L.qb[j] = (int)(q % 64);
+        }
+        L.pattern_mask = (1u << (2 * t.k)) - 1u;
+        for (int w = 0; w < W; ++w) {
+            L.gx[w] = t.entries[e].mask_x[w];
+            L.gz[w] = t.entries[e].mask_z[w];
+        }
+        st.undo = L;
+        for (int s = 0; s < 16; ++s) {
+            const bool in = s < dim, moves = in && delta[s] == g;
+            // patterns that stay for good take their sign with the first step
+            const double a0 = moves ? 0.0 : (in && delta[s] == 0 && steps.size() == 1 ? amp[s] : 1.0);
+            L.a0[s] = st.undo.a0[s] = a0;
+            L.a1[s] = moves ? amp[s] : 0.0;
+            st.undo.a1[s] = moves ? amp[s ^ g] : 0.0;
+            L.a0f[s] = st.undo.a0f[s] = (float)a0;
+            L.a1f[s] = (float)L.a1[s];
+            st.undo.a1f[s] = (float)st.undo.a1[s];
+        }
+        st.lv.n = 0;
+        for (int half = 0; half < 2; ++half)
+            for (int w = 0; w < W; ++w) {
+                uint64_t bits = half ? L.gz[w] : L.gx[w];
+                while (bits) {
+                    const int b = 63 - __builtin_clzll(bits);
+                    st.lv.rank[st.lv.n++] = (uint32_t)(64 * (half ? W + w : w) + (63 - b));
+                    bits &= ~(1ull << b);
+                }
+            }
+    }
+    return !steps.empty();
+}
+
 // A local table as per-pattern record lists (ascending entry order, zero amplitudes in the
 // coefficient type skipped, as DeltaEntry::emit skips them).
 template <int W, typename T>
@@ -1242,7 +1323,11 @@ struct Engine {
     // noise (optional): single-qubit key-preserving channels to fold in before the table, in
     // order; noise_after[j] receives the terms left after channel j.
     static ps_status apply(ps_sum* s, const ps_table& t, const ps_policy* policy, ps_layer_stats* stats,
-                           const NoiseList* noise = nullptr, uint64_t* noise_after = nullptr) {
+                           const NoiseList* noise = nullptr, uint64_t* noise_after = nullptr,
+                           const PermStep<W>* step = nullptr, const RotLayer<W>* step_L = nullptr, bool inner = false) {
+        // step: one step of the table's permutation (step_L: its layer or the one that takes it back);
+        // inner: not its last, so neither the keep program nor the policy's passes see it
+        if (inner) policy = nullptr;
         KeepProg keep;
         std::string why;
         // the last TopN pass wrote this layer's partner list (the store is as it left it)
@@ -1256,8 +1341,13 @@ struct Engine {
         RotationArgs<W, T> a;
         std::memset(&a, 0, sizeof a);
         bool general = false;
-        ps = to_rot_layer<W, T>(t, a.L, *s->levels, why, &general);
-        if (ps != PS_OK) return set_err(s, ps, why);
+        if (step) {
+            a.L = *step_L;
+            *s->levels = step->lv;
+        } else {
+            ps = to_rot_layer<W, T>(t, a.L, *s->levels, why, &general);
+            if (ps != PS_OK) return set_err(s, ps, why);
+        }
         uint64_t lsup[W];
         table_support<W>(t, lsup);
         if (general) return apply_general(s, t, keep, policy, stats, lsup);
@@ -1265,7 +1355,7 @@ struct Engine {
             // a commuting term keeps c exactly on the wide path; a local table must leave the
             // identity pattern alone
             const bool identity0 = a.L.wide || ((T)a.L.a1[0] == T(0) && (T)a.L.a0[0] == T(1));
-            if (!noise && skippable(s, lsup, keep, identity0)) {
+            if (!noise && !step && skippable(s, lsup, keep, identity0)) {
                 skipped(s, stats, a.L.partners ? PS_PATH_ROTATION : PS_PATH_RESCALE);
                 return PS_OK;
             }
@@ -1273,7 +1363,7 @@ struct Engine {
         const uint64_t n = cut_in ? s->cut_rows : s->n;
         if (n >= (1ull << 31) - 1) return set_err(s, PS_ERR_UNSUPPORTED, "apply: at most 2^31 - 2 terms");
         const int spare = 1 - s->cur;
-        const uint64_t out_rows = cut_in ? n + s->cut_m : a.L.partners ? 2 * n : n;
+        const uint64_t out_rows = step ? n : cut_in ? n + s->cut_m : a.L.partners ? 2 * n : n;
         // the first layer pass is TopN (or ApproxTopN) and could trigger: the merge builds its
         // first select digit (the octave histogram); before plain TopN the merge writes slots
         const int first_pass = policy && policy->num_passes > 0 ? policy->passes[0].kind : PS_PASS_NONE;
@@ -1283,7 +1373,7 @@ struct Engine {
         const bool scored_fuse = carry_f && first_pass == PS_PASS_SCORED_TOPN;
         const bool fuse_topn = (first_pass == PS_PASS_TOPN || first_pass == PS_PASS_APPROX_TOPN || scored_fuse) &&
                                out_rows > policy->passes[0].n;
-        const uint64_t span_rows = merge_span_rows<W>(out_rows);
+        const uint64_t span_rows = merge_span_rows<W>(step ? 2 * n : out_rows);
         // (the TopN kernels index a slotted store's rows in 32 bits)
         const bool slotted = fuse_topn && (first_pass == PS_PASS_TOPN || scored_fuse) && !s->fault_stall &&
                              span_rows < (1ull << 32);
@@ -1337,7 +1427,7 @@ struct Engine {
             a.cut_pr = (uint32_t*)s->cut_pr.p;
             a.cut_bslot = (uint4*)s->cut_bslot.p;
         }
-        const uint64_t tiles_hi = out_rows / kMinTileRows + 4;
+        const uint64_t tiles_hi = (step ? 2 * n : out_rows) / kMinTileRows + 4;
         if ((e = ensure(s, s->status, tiles_hi * sizeof(unsigned long long))) != cudaSuccess ||
             (e = ensure(s, s->bounds, (tiles_hi + 2) * sizeof(ulonglong2))) != cudaSuccess)
             return cuda_fail(s, e, "apply: scratch");
@@ -1582,6 +1672,7 @@ struct Engine {
             uint64_t lsup[W];
         };
         std::vector<Entry> entries;
+        std::vector<PermStep<W>> perm;
         std::vector<RunLayer<W, T>> prog;
         std::vector<T> noise_f;
         std::vector<uint16_t> noise_q;
@@ -1619,21 +1710,27 @@ struct Engine {
                     s->levels->n <= kRunLevels)
                     at = fj;
             }
+            perm.clear();
             if (at == c) {
                 general = false;
-                if (to_rot_layer<W, T>(tables[c], R, *s->levels, why, &general) != PS_OK || general) break;
-                if (R.partners && s->levels->n > kRunLevels) break;
+                if (to_rot_layer<W, T>(tables[c], R, *s->levels, why, &general) != PS_OK) break;
+                if (general && !permutation_steps<W, T>(tables[c], perm)) break;
+                if (!general && R.partners && s->levels->n > kRunLevels) break;
                 // noise cut off from its rotation by the end of the run is left to the next one
                 if (fj > c && fj == end && end < ntables) break;
             }
             table_support<W>(tables[at], en.lsup);
             en.channels = at - c + 1;
-            en.partners = R.partners != 0;
+            en.partners = R.partners != 0 || !perm.empty();
             en.prog = -1;
-            const bool identity0 = R.wide || ((T)R.a1[0] == T(0) && (T)R.a0[0] == T(1));
+            const bool identity0 = !perm.empty() || R.wide || ((T)R.a1[0] == T(0) && (T)R.a0[0] == T(1));
             bool skip = at == c && identity0 && clean;
             for (int w = 0; w < W; ++w) skip = skip && !(en.lsup[w] & sup[w]);
-            if (!skip) {
+            for (size_t part = 0; !skip && part < std::max<size_t>(1, perm.size()); ++part) {
+                if (!perm.empty()) {
+                    R = perm[part].L;
+                    *s->levels = perm[part].lv;
+                }
                 RunLayer<W, T> P;
                 std::memset(&P, 0, sizeof P);
                 for (int w = 0; w < W; ++w) {
@@ -1665,9 +1762,13 @@ struct Engine {
                     noise_q.push_back((uint16_t)tables[q].qubits[0]);
                     for (int z = 0; z < 4; ++z) noise_f.push_back((T)tables[q].entries[0].amplitude[z]);
                 }
+                P.inner = part + 1 < perm.size() ? 1 : 0;
+                P.group = part == 0 ? (int32_t)perm.size() : 0;
                 en.prog = (int32_t)prog.size();
                 prog.push_back(P);
-                if (R.partners) {
+                if (!perm.empty()) {
+                    for (int w = 0; w < W; ++w) sup[w] |= en.lsup[w];
+                } else if (R.partners) {
                     grow = std::min<uint64_t>(2 * grow, room);
                     for (int w = 0; w < W; ++w) sup[w] |= en.lsup[w];
                 }
@@ -1811,11 +1912,35 @@ struct Engine {
         return PS_OK;
     }
 
+    // A signed permutation, step by step.  Its steps after the first allocate nothing (a step adds no
+    // row); one that fails takes the ones before it back, so the store keeps the last completed layer.
+    static ps_status apply_permutation(ps_sum* s, const ps_table& t, const std::vector<PermStep<W>>& steps,
+                                       const ps_policy* policy, ps_layer_stats* stats) {
+        const uint64_t n = terms_of(s);
+        for (size_t i = 0; i < steps.size(); ++i) {
+            const bool last = i + 1 == steps.size();
+            ps_layer_stats ls;
+            ps_status ps = apply(s, t, policy, last ? stats : &ls, nullptr, nullptr, &steps[i], &steps[i].L, !last);
+            if (ps == PS_OK) continue;
+            const std::string err = s->err;
+            for (size_t j = i; j-- > 0;)
+                if (apply(s, t, nullptr, &ls, nullptr, nullptr, &steps[j], &steps[j].undo, true) != PS_OK) break;
+            s->keep_clean = false;
+            s->err = err;
+            return ps;
+        }
+        if (stats) {
+            stats->terms_in = n;
+            stats->partners = 0;
+            stats->path = PS_PATH_SORT;
+        }
+        return PS_OK;
+    }
+
     // The sort path: branch records, LSD radix sort of (key, record index), run-summing dedup
     // with the keep program (apply_layer_body's general tables, engine/gpu/layer.rs:614-763).
     static ps_status apply_general(ps_sum* s, const ps_table& t, const KeepProg& keep, const ps_policy* policy,
                                    ps_layer_stats* stats, const uint64_t (&lsup)[W]) {
-        (void)policy;
         GenLayer<W, T> G;
         to_gen_layer<W, T>(t, G);
         s->f_valid = false;  // the sort path carries no predictions
@@ -1827,6 +1952,10 @@ struct Engine {
                 skipped(s, stats, PS_PATH_SORT);
                 return PS_OK;
             }
+        }
+        {
+            std::vector<PermStep<W>> steps;
+            if (permutation_steps<W, T>(t, steps)) return apply_permutation(s, t, steps, policy, stats);
         }
         const uint64_t n = s->n;
         if (s->hist_ready) {

@@ -100,7 +100,8 @@ struct LevelList {
 template <int W>
 struct RotLayer {
     uint64_t gx[W], gz[W];   // partner delta (generator) x / z masks
-    int32_t wide;            // 1: PreparedRotation (per-term phase), 0: LocalPtm lookup
+    int32_t wide;            // 1: PreparedRotation (per-term phase), 0: LocalPtm lookup, 2: one step of a
+                             // permutation (a pattern with a1 != 0 moves: a0 is 0 and no own row stays)
     int32_t partners;        // 0: key-preserving, no partner stream
     int32_t qw[2], qb[2];    // support qubit j lives in word qw[j], bit qb[j]
     uint32_t pattern_mask;   // (1 << 2k) - 1

@@ -1081,7 +1081,8 @@ cudaError_t launch_rotation_layer(const RotationArgs<W, T>& a, cudaStream_t st) 
         *a.out_count = 0;
         return cudaSuccess;
     }
-    if ((a.slot_count ? (uint64_t)mtiles_hi * (MT + 2) : total_hi) > a.out_cap) return cudaErrorMemoryAllocation;
+    const uint64_t rows_hi = a.L.wide == 2 ? a.n : total_hi;  // a permutation's step adds no row
+    if ((a.slot_count ? (uint64_t)mtiles_hi * (MT + 2) : rows_hi) > a.out_cap) return cudaErrorMemoryAllocation;
     if (a.cut) {
         const CutStore S{a.cut_pr, a.cut_tiles, a.cut->slot_rows};
         if ((e = CutOps<W, T>::partition(a.Sk, a.n, S, a.Pk, a.cut_m, (uint32_t)MT, a.bounds, a.cut_bslot, a.sms, st,

@@ -76,7 +76,7 @@ __device__ __forceinline__ void stage_amps(const RotLayer<W>& L, AmpTab<T>& t) {
 template <int W, typename T, typename LT>
 __device__ __forceinline__ bool emits_partner_regs(const LT& L, const AmpTab<T>& A,
                                                    const uint64_t (&k)[2 * W]) {
-    if (L.wide) {
+    if (L.wide == 1) {
         uint64_t f = 0;
 #pragma unroll
         for (int i = 0; i < W; ++i) f ^= (k[i] & L.gz[i]) ^ (k[W + i] & L.gx[i]);
@@ -99,14 +99,18 @@ __device__ __forceinline__ uint32_t div_regs(const uint64_t (&a)[2 * W], const u
 // Own-row coefficient after the layer.
 template <int W, typename T, typename LT>
 __device__ __forceinline__ T own_coeff(const LT& L, const AmpTab<T>& A, const uint64_t* k, T c) {
-    if (L.wide) return anticommutes<W>(k, L.gx, L.gz) ? mul_rn(c, Amp<T>::cs(L)) : c;
+    if (L.wide) {
+        if (L.wide == 1) return anticommutes<W>(k, L.gx, L.gz) ? mul_rn(c, Amp<T>::cs(L)) : c;
+        const T a = A.a0[pattern_of<W>(L, k)];  // a moved row leaves nothing, whatever its coefficient
+        return a == T(0) ? T(0) : mul_rn(c, a);
+    }
     return mul_rn(c, A.a0[pattern_of<W>(L, k)]);
 }
 
 // Partner coefficient (DeltaEntry::emit / PreparedRotation::emit_generator).
 template <int W, typename T, typename LT>
 __device__ __forceinline__ T partner_coeff(const LT& L, const AmpTab<T>& A, const uint64_t* k, T c) {
-    if (L.wide) {
+    if (L.wide == 1) {
         uint32_t total = (1u + product_phase<W>(k, L.gx, L.gz)) & 3u;
         T m = (total & 2u) ? -c : c;  // real mul_phase, coefficient.rs:107-114
         return mul_rn(m, Amp<T>::sn(L));

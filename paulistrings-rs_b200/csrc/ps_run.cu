@@ -511,7 +511,9 @@ __global__ void __launch_bounds__(kRunThreads, 1) k_layer_run(const RunArgs<W, T
         const uint64_t n = s_n, m = s_m;
         const uint32_t tile = (uint32_t)((n + m + G - 1) / G);
         // every block takes the same decision: the layer fits the blocks and the buffers, or the run ends
-        const bool fits = tile + 1 <= a.rcap && n <= a.wcap && m <= a.pcap;
+        // (a permutation's later steps take at most the same rows again)
+        const uint32_t most = !done && L.group > 1 ? (uint32_t)((2 * n + G - 1) / G) : tile;
+        const bool fits = most + 1 <= a.rcap && n <= a.wcap && m <= a.pcap;
         // the rows at their positions
         {
             unsigned int r = s_off + ra;
@@ -662,6 +664,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) k_layer_run(const RunArgs<W, T
         }
         __syncthreads();
         unsigned int alive = 0;
+        const bool inner = L.inner != 0;
         {
             uint32_t i = s_si[tid], j = s_sj[tid];
             const uint32_t ie = s_si[tid + 1], je = s_sj[tid + 1];
@@ -690,12 +693,12 @@ __global__ void __launch_bounds__(kRunThreads, 1) k_layer_run(const RunArgs<W, T
                         S.src[q + 1] = kDead;  // the pair's second slot
                         if (++j < je) ld_row<W>(sPk, j, y);
                     }
-                    ok = v != T(0) && keep_eval<W>(a.keep, x, to_f64(v));
+                    ok = v != T(0) && (inner || keep_eval<W>(a.keep, x, to_f64(v)));
                     if (++i < ie) ld_row<W>(S.key, i, x);
                 } else {
                     src = (uint16_t)(cs_ + j);
                     v = S.c[cs_ + j];
-                    ok = v != T(0) && keep_eval<W>(a.keep, y, to_f64(v));
+                    ok = v != T(0) && (inner || keep_eval<W>(a.keep, y, to_f64(v)));
                     if (++j < je) ld_row<W>(sPk, j, y);
                 }
                 S.src[q] = ok ? src : kDead;
@@ -708,7 +711,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) k_layer_run(const RunArgs<W, T
         if (nnoise)
             for (int i = tid; i < nnoise; i += kRunThreads)
                 if (s_drop[i]) atomicAdd(&a.drops[L.noise_first + i], s_drop[i]);
-        if (a.topn == 0 || n + m <= a.topn) {
+        if (a.topn == 0 || n + m <= a.topn || L.wide == 2) {  // (a permutation adds no row)
             if (a.topn) count_rows(alive, &a.after_rows[layer]);
             continue;
         }

@@ -29,7 +29,8 @@ struct alignas(16) RunLayer {
     int32_t nlev;
     uint32_t rank[kRunLevels];
     int32_t noise_first, noise_n;  // folded noise: its channels' place in the run's noise tables
-    int32_t pad[2];
+    int32_t inner;                 // a permutation's step before its last: no keep program
+    int32_t group;                 // steps of the permutation that starts here (they run or stop together)
 };
 
 // A block's part of a layer, read by every block after the layer's first barrier.
